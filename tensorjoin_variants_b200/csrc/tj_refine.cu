@@ -25,21 +25,41 @@ namespace tj {
 namespace {
 
 // ------------------------------------------------------------------ plain FP32 join
+// A unit is 128 R rows x 64 S rows (a quarter of a candidate tile pair); a CTA of 16 x 16 threads
+// holds 8 x 4 pairs per thread, each as two running sums (even and odd k) in one FP32x2 register
+// pair, so a row's (k, k + 1) read from shared memory is a packed operand as it lies there.
+//
+// What bounds it: FP32 issue (a packed subtract and a packed FMA per two elements of a pair; the
+// packed pipe alone needs 180 us for the 202M pairs of a 20,000 x 16 self-join), with the per-pair
+// sum and classification on top of it below d = 16.  The form this replaces took 31,000 cycles per
+// 128 x 256 tile pair at d = 16 and at d = 2 alike (8 x 16 pairs per thread and one CTA per SM: the
+// latency of unpipelined loads and a branch per pair).  Hence two CTAs of 8 warps per SM, operand
+// chunks brought in two stages ahead by cp.async (across unit and tile borders), one minimum over a
+// thread's 32 pairs in front of the per-pair tests, and an even cut of all units over the CTAs
+// (chunks of 64 tile pairs left half of them idle on 20,000 rows).  Measured (one B200): 20,000 x 16
+// self-join 702 -> 376 us; 100,000 x 2 self-join with 13.7M pairs 643 -> 290 us.
 constexpr int kPT = 256;                // threads: 16 x 16
-constexpr int kPR = 8, kPC = 16;        // micro-tile: 8 rows x 16 cols per thread
-constexpr int kPK = 16;                 // k chunk
+constexpr int kPI = 8, kPJ = 4;         // pairs per thread: rows i * 16 + ty, columns j * 16 + tx
+constexpr int kPCols = 64;              // columns of a unit
+constexpr int kPUnits = kTileS / kPCols;
+constexpr int kPK = 16;                 // k chunk (elements per stage)
+constexpr int kPLd = kPK + 4;           // shared row stride: 16-byte reads of 8 rows hit distinct banks
+constexpr int kPStages = 3;
+constexpr int kPRows = kTileR + kPCols; // staged rows: R tile, then the unit's S rows
 
 struct PlainClass {
-    const float* rx;     // [rows_pad, d] sorted FP32 rows (R side of the class)
-    const float* sx;     // [rows_pad, d] sorted FP32 rows (S side)
+    const float* rx;     // [rows, d] FP32 rows (R side of the class)
+    const float* sx;     // [rows, d] FP32 rows (S side)
     const uint32_t* r_emit;
     const uint32_t* s_emit;
     int d;
+    int vec;             // rows are multiples of 16 bytes, 16-byte aligned
 };
 
 struct PlainArgs {
-    const uint4* chunks;
-    const uint32_t* nchunks;
+    const uint32_t* off;        // [ntR] first candidate of each R tile
+    const uint32_t* total;      // candidates
+    int ntR;
     const uint32_t* jlist;
     const uint4* rtiles;        // (row0, nvalid, join, class) per global R tile
     const uint4* stiles;
@@ -53,114 +73,271 @@ struct PlainArgs {
     Counters* ctr;
 };
 
-// a0 += (r - s0)^2, a1 += (r - s1)^2 as one packed FP32x2 subtract and one packed FP32x2 FMA (sm_100);
-// each lane is rounded exactly as the scalar subtract and fmaf
-TJ_DEV void sqdiff_acc_x2(float r, float s0, float s1, float& a0, float& a1) {
-    asm("{\n\t.reg .b64 x, y, t, c;\n\t"
-        "mov.b64 x, {%2, %2};\n\t"
-        "mov.b64 y, {%3, %4};\n\t"
-        "mov.b64 c, {%0, %1};\n\t"
-        "sub.rn.f32x2 t, x, y;\n\t"
-        "fma.rn.f32x2 c, t, t, c;\n\t"
-        "mov.b64 {%0, %1}, c;\n\t}"
-        : "+f"(a0), "+f"(a1) : "f"(r), "f"(s0), "f"(s1));
+TJ_DEV void cp_async4_zfill(void* dst, const void* src, bool real) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                 :: "r"(smem_u32(dst)), "l"((uint64_t)src), "r"(real ? 4u : 0u) : "memory");
+}
+// acc += (r - s)^2 in both halves, each rounded as the scalar subtract and fmaf
+TJ_DEV void sqdiff_x2(unsigned long long r, unsigned long long s, unsigned long long& acc) {
+    asm("{\n\t.reg .b64 t;\n\t"
+        "sub.rn.f32x2 t, %1, %2;\n\t"
+        "fma.rn.f32x2 %0, t, t, %0;\n\t}"
+        : "+l"(acc) : "l"(r), "l"(s));
+}
+TJ_DEV float sum_x2(unsigned long long v) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return lo + hi;
 }
 
-__global__ void __launch_bounds__(kPT, 1) plain_kernel(const PlainArgs a) {
-    __shared__ float sR[kPK][kTileR + 1];   // +1: conflict-free transposed stores
-    __shared__ float sS[kPK][kTileS + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const unsigned nchunks = *a.nchunks;
-    WarpAppender app_acc, app_band;
-    unsigned long long n_items = 0, n_screen_acc = 0;
-    for (unsigned c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint4 ch = a.chunks[c];
-        const uint4 rt = a.rtiles[ch.x];
-        const PlainClass& pc = a.cls[rt.w];
-        const JoinParams jp = a.jps[rt.z];
-        const float2 th = a.thr[rt.z];
-        const int d = pc.d;
-        const unsigned r0 = rt.x, nvI = rt.y;
-        for (unsigned e = ch.y; e < ch.z; ++e) {
-            const unsigned J = a.jlist[e];
-            const uint4 stt = a.stiles[J];
-            const unsigned c0 = stt.x, nvJ = stt.y;
-            float acc[kPR][kPC];
-#pragma unroll
-            for (int i = 0; i < kPR; ++i)
-#pragma unroll
-                for (int j = 0; j < kPC; ++j) acc[i][j] = 0.f;
-            for (int k0 = 0; k0 < d; k0 += kPK) {
-                __syncthreads();
-                for (int idx = threadIdx.x; idx < kPK * kTileR; idx += kPT) {
-                    const int r = idx / kPK, k = idx % kPK;
-                    sR[k][r] = (k0 + k < d) ? pc.rx[(size_t)(r0 + r) * d + k0 + k] : 0.f;
-                }
-                for (int idx = threadIdx.x; idx < kPK * kTileS; idx += kPT) {
-                    const int r = idx / kPK, k = idx % kPK;
-                    sS[k][r] = (k0 + k < d) ? pc.sx[(size_t)(c0 + r) * d + k0 + k] : 0.f;
-                }
-                __syncthreads();
-                const int kmax = min(kPK, d - k0);
-                for (int k = 0; k < kmax; ++k) {
-                    float rv[kPR], sv[kPC];
-#pragma unroll
-                    for (int i = 0; i < kPR; ++i) rv[i] = sR[k][i * 16 + ty];   // rows i*16+ty, cols j*16+tx
-#pragma unroll
-                    for (int j = 0; j < kPC; ++j) sv[j] = sS[k][j * 16 + tx];
-#pragma unroll
-                    for (int i = 0; i < kPR; ++i)
-#pragma unroll
-                        for (int j = 0; j < kPC; j += 2)
-                            sqdiff_acc_x2(rv[i], sv[j], sv[j + 1], acc[i][j], acc[i][j + 1]);
-                }
-            }
-            // classify: groups of 32 pairs (2 rows x 16 cols) so that emission stays warp-uniform
-#pragma unroll
-            for (int g = 0; g < kPR / 2; ++g) {
-                uint32_t amask = 0, bmask = 0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int j = 0; j < kPC; ++j) {
-                        const int i = g * 2 + h;
-                        const unsigned row = i * 16 + ty, col = j * 16 + tx;
-                        const float s = acc[i][j];
-                        if (s > th.y || row >= nvI || col >= nvJ) continue;
-                        if (jp.self_join && c0 + col <= r0 + row) continue;
-                        if (s <= th.x) amask |= 1u << (h * 16 + j);
-                        else bmask |= 1u << (h * 16 + j);
-                    }
-                unsigned ta, tb;
-                const unsigned pa = warp_excl_scan(__popc(amask), ta);
-                const unsigned pb = warp_excl_scan(__popc(bmask), tb);
-                if (ta) {
-                    unsigned long long pos = app_acc.reserve(ta, &a.ctr->acc_reserved, a.acc, a.acc_cap) + pa;
-                    uint32_t mk = amask;
-                    while (mk) {
-                        const int b = __ffs(mk) - 1;
-                        mk &= mk - 1;
-                        const unsigned row = (g * 2 + (b >> 4)) * 16 + ty, col = (b & 15) * 16 + tx;
-                        if (pos < a.acc_cap) a.acc[pos] = pair_key(jp, pc.r_emit[r0 + row], pc.s_emit[c0 + col]);
-                        ++pos;
-                    }
-                    n_screen_acc += __popc(amask);
-                }
-                if (tb) {
-                    unsigned long long pos = app_band.reserve(tb, &a.ctr->band_reserved, a.band, a.band_cap) + pb;
-                    uint32_t mk = bmask;
-                    while (mk) {
-                        const int b = __ffs(mk) - 1;
-                        mk &= mk - 1;
-                        const unsigned row = (g * 2 + (b >> 4)) * 16 + ty, col = (b & 15) * 16 + tx;
-                        if (pos < a.band_cap) a.band[pos] = pair_key(jp, pc.r_emit[r0 + row], pc.s_emit[c0 + col]);
-                        ++pos;
-                    }
-                }
-            }
-            ++n_items;
-        }
+// What the compute side needs to know of a stage (written by thread 0 when the stage is issued).
+struct PlainStage {
+    unsigned r0, nvI, c0, nvJ;   // rows of the R tile, columns of the unit
+    unsigned join;
+    int kc;                      // elements in the stage (0: no more stages)
+    int first, last;             // first / last k chunk of the unit
+    float2 th;                   // the join's thresholds
+};
+
+// R tile of candidate e: the last one whose first candidate is <= e (warp-collective).
+TJ_DEV int find_rtile(const uint32_t* off, int n, uint32_t e) {
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) / 32;
+        const int p = lo + (int)lane_id() * step;
+        const unsigned m = __ballot_sync(0xffffffffu, p < hi && off[p] <= e);   // lane 0 always passes
+        lo += (31 - __clz(m)) * step;
+        hi = min(hi, lo + step);
     }
+    return lo;
+}
+
+__global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
+    __shared__ __align__(16) float sm[kPStages][kPRows][kPLd];
+    __shared__ PlainStage info[kPStages];
+    __shared__ uint32_t ids[kPStages][kPRows];   // emitted row ids of the unit's rows and columns
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // this CTA's run of all candidates' quarters, in candidate order: candidate e, quarter p, `left` units
+    const unsigned long long units = (unsigned long long)*a.total * kPUnits;
+    const unsigned long long u0 = units * blockIdx.x / gridDim.x;
+    unsigned left = (unsigned)(units * (blockIdx.x + 1) / gridDim.x - u0);
+    uint32_t e = (uint32_t)(u0 / kPUnits);
+    unsigned p = (unsigned)(u0 % kPUnits) * kPCols;
+    __shared__ WarpAppender apps[kPT / 32][2];   // accept and band of each warp: touched by hits only
+    WarpAppender* app = apps[threadIdx.x >> 5];
+    if (lane_id() < 2) app[lane_id()] = WarpAppender();
+    __syncwarp();
+    unsigned n_screen_acc = 0, n_items = 0;
+
+    // issue side: the stage that comes next
+    int k0 = 0;
+    uint32_t e_end = 0;   // first candidate beyond the R tile of the last one (0: no tile yet)
+    bool fresh = true;    // candidate e's tiles are not taken yet
+    uint4 rt = make_uint4(0, 0, 0, 0);
+    // the S tile (first row, rows) of candidate e, and the next one's, whose two dependent loads are
+    // issued a quarter apart so that neither is waited for
+    uint2 stt = make_uint2(0, 0), stn = stt;
+    uint32_t jn = 0;
+    const uint32_t total = *a.total;
+    bool self_join = false, first = true;
+    float2 th = make_float2(0.f, 0.f);
+    auto s_tile = [&](uint32_t j) { return *reinterpret_cast<const uint2*>(a.stiles + j); };
+    const float *pr0 = nullptr, *pr1 = nullptr, *ps = nullptr;   // 16-byte copies: this thread's R and S elements
+    const unsigned lr = threadIdx.x >> 2, lq = (threadIdx.x & 3) * 4;
+    auto step = [&] {
+        --left;
+        p += kPCols;
+        if (p == (unsigned)kTileS) {
+            p = 0;
+            ++e;
+            fresh = true;
+        }
+    };
+    auto issue = [&](int buf) {
+        // the unit's tiles (units without a column, or at or below a self-join's diagonal, are passed over)
+        while (k0 == 0 && left) {
+            if (fresh) {
+                fresh = false;
+                if (e >= e_end) {
+                    const int I = find_rtile(a.off, a.ntR, e);
+                    e_end = I + 1 < a.ntR ? a.off[I + 1] : 0xFFFFFFFFu;
+                    rt = a.rtiles[I];
+                    // rows past a tile's points repeat its last one, so no read leaves the side
+                    const PlainClass& pc = a.cls[rt.w];
+                    pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.d + lq;
+                    pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.d + lq;
+                    self_join = a.jps[rt.z].self_join != 0;
+                    th = a.thr[rt.z];
+                }
+                stt = stn;
+                if (first) {
+                    first = false;
+                    stt = s_tile(a.jlist[e] & kJMask);
+                    if (p != 0) jn = a.jlist[min(e + 1, total - 1)] & kJMask;
+                }
+            }
+            if (p == 0) {
+                ++n_items;
+                jn = a.jlist[min(e + 1, total - 1)] & kJMask;
+            }
+            if (p == kTileS - kPCols) stn = s_tile(jn);
+            if (p < stt.y && !(self_join && stt.x + p + kPCols <= rt.x + 1)) break;
+            step();
+        }
+        if (!left) {
+            if (threadIdx.x == 0) info[buf].kc = 0;
+            cp_async_commit();
+            return;
+        }
+        const unsigned c0 = stt.x + p, nvJ = min(stt.y - p, (unsigned)kPCols);
+        const PlainClass& pc = a.cls[rt.w];
+        const int d = pc.d, kc = min(kPK, d - k0);
+        if (pc.vec) {
+            if (k0 == 0) ps = pc.sx + (size_t)(c0 + min(lr, nvJ - 1)) * d + lq;
+            if ((int)lq < kc) {
+                cp_async16(&sm[buf][lr][lq], pr0 + k0);
+                cp_async16(&sm[buf][lr + 64][lq], pr1 + k0);
+                cp_async16(&sm[buf][kTileR + lr][lq], ps + k0);
+            }
+        } else {   // elements up to the next power of two, zero beyond kc
+            const int lk = kc <= 2 ? 1 : kc <= 4 ? 2 : kc <= 8 ? 3 : 4;
+            for (int idx = threadIdx.x; idx < kPRows << lk; idx += kPT) {
+                const int r = idx >> lk, k = idx & ((1 << lk) - 1);
+                const float* row = r < kTileR ? pc.rx + (size_t)(rt.x + min((unsigned)r, rt.y - 1)) * d
+                                              : pc.sx + (size_t)(c0 + min((unsigned)(r - kTileR), nvJ - 1)) * d;
+                cp_async4_zfill(&sm[buf][r][k], row + k0 + min(k, kc - 1), k < kc);
+            }
+        }
+        if (threadIdx.x == 0)
+            info[buf] = PlainStage{rt.x, rt.y, c0, nvJ, rt.z, kc, k0 == 0, k0 + kc >= d, th};
+        if (k0 + kc >= d && threadIdx.x < kPRows) {
+            const unsigned t = threadIdx.x;
+            cp_async4_zfill(&ids[buf][t], t < kTileR ? pc.r_emit + rt.x + min(t, rt.y - 1)
+                                                     : pc.s_emit + c0 + min(t - kTileR, nvJ - 1), true);
+        }
+        k0 += kPK;
+        if (k0 >= d) {
+            k0 = 0;
+            step();
+        }
+        cp_async_commit();
+    };
+
+    unsigned long long acc[kPI][kPJ];
+    issue(0);
+    issue(1);
+    for (int buf = 0;; buf = buf == kPStages - 1 ? 0 : buf + 1) {
+        cp_async_wait<1>();
+        __syncthreads();   // this stage has landed and the one before it is no longer read
+        const PlainStage in = info[buf];
+        if (in.kc == 0) break;
+        issue(buf == 0 ? kPStages - 1 : buf - 1);
+        if (in.first) {
+#pragma unroll
+            for (int i = 0; i < kPI; ++i)
+#pragma unroll
+                for (int j = 0; j < kPJ; ++j) acc[i][j] = 0ull;
+        }
+        const float(&sR)[kPRows][kPLd] = sm[buf];
+        const float(*sS)[kPLd] = sm[buf] + kTileR;
+        const int quads = (in.kc + 1) >> 2;   // 3 left over: a whole quad (its last element is 0 on both sides)
+        for (int q = 0; q < quads; ++q) {
+            ulonglong2 sv[kPJ];
+#pragma unroll
+            for (int j = 0; j < kPJ; ++j) sv[j] = *reinterpret_cast<const ulonglong2*>(&sS[j * 16 + tx][q * 4]);
+#pragma unroll
+            for (int i = 0; i < kPI; ++i) {
+                const ulonglong2 rv = *reinterpret_cast<const ulonglong2*>(&sR[i * 16 + ty][q * 4]);
+#pragma unroll
+                for (int j = 0; j < kPJ; ++j) {
+                    sqdiff_x2(rv.x, sv[j].x, acc[i][j]);
+                    sqdiff_x2(rv.y, sv[j].y, acc[i][j]);
+                }
+            }
+        }
+        if (in.kc > quads * 4) {   // one or two elements left over
+            unsigned long long sv[kPJ];
+#pragma unroll
+            for (int j = 0; j < kPJ; ++j)
+                sv[j] = *reinterpret_cast<const unsigned long long*>(&sS[j * 16 + tx][quads * 4]);
+#pragma unroll
+            for (int i = 0; i < kPI; ++i) {
+                const unsigned long long rv = *reinterpret_cast<const unsigned long long*>(&sR[i * 16 + ty][quads * 4]);
+#pragma unroll
+                for (int j = 0; j < kPJ; ++j) sqdiff_x2(rv, sv[j], acc[i][j]);
+            }
+        }
+        if (!in.last) continue;
+        // classify the thread's 32 pairs: bit i * kPJ + j
+        
+        float v[kPI * kPJ];
+#pragma unroll
+        for (int b = 0; b < kPI * kPJ; ++b) v[b] = sum_x2(acc[b / kPJ][b % kPJ]);
+        // least sum of each of the thread's rows: one vote while no pair is near the threshold, then the
+        // rows that hold a near pair in some lane, and only their pairs one by one
+        float rm[kPI];
+#pragma unroll
+        for (int i = 0; i < kPI; ++i) rm[i] = fminf(fmin3(v[i * kPJ], v[i * kPJ + 1], v[i * kPJ + 2]), v[i * kPJ + 3]);
+        const float m = fmin3(fmin3(rm[0], rm[1], rm[2]), fmin3(rm[3], rm[4], rm[5]), fminf(rm[6], rm[7]));
+        if (!__any_sync(0xffffffffu, !(m > in.th.y))) continue;
+        unsigned rows = 0;
+#pragma unroll
+        for (int i = 0; i < kPI; ++i) rows |= rm[i] > in.th.y ? 0u : 1u << i;
+        rows = __reduce_or_sync(0xffffffffu, rows);
+        uint32_t cand = 0, amask = 0;
+#pragma unroll
+        for (int i = 0; i < kPI; ++i) {
+            if (!(rows & (1u << i))) continue;
+#pragma unroll
+            for (int b = i * kPJ; b < (i + 1) * kPJ; ++b) {
+                cand |= v[b] > in.th.y ? 0u : 1u << b;
+                amask |= v[b] <= in.th.x ? 1u << b : 0u;
+            }
+        }
+        // valid rows and columns of this thread
+        const int ni = min(max((int)in.nvI - ty + 15, 0) >> 4, kPI), nj = min(max((int)in.nvJ - tx + 15, 0) >> 4, kPJ);
+        const uint32_t rmask = ni == kPI ? 0xFFFFFFFFu : (1u << (kPJ * ni)) - 1u;
+        cand &= rmask & (((1u << nj) - 1u) * 0x11111111u);
+        const JoinParams& jp = a.jps[in.join];
+        if (jp.self_join && in.c0 <= in.r0 + kTileR - 1) {   // keep sorted column > sorted row only
+            uint32_t w = cand;
+            while (w) {
+                const int b = __ffs(w) - 1;
+                w &= w - 1;
+                if (in.c0 + (b % kPJ) * 16 + tx <= in.r0 + (b / kPJ) * 16 + ty) cand &= ~(1u << b);
+            }
+        }
+        amask &= cand;
+        const uint32_t bmask = cand & ~amask;
+        unsigned tot;
+        const unsigned pre = warp_excl_scan(__popc(amask) | (__popc(bmask) << 16), tot);
+        const unsigned ta = tot & 0xFFFFu, tb = tot >> 16;
+        auto put = [&](uint32_t w, uint64_t* out, unsigned long long pos, unsigned long long cap) {
+            while (w) {
+                const int b = __ffs(w) - 1;
+                w &= w - 1;
+                const uint32_t oi = ids[buf][(b / kPJ) * 16 + ty], oj = ids[buf][kTileR + (b % kPJ) * 16 + tx];
+                if (pos < cap) out[pos] = pair_key(jp, oi, oj);
+                ++pos;
+            }
+        };
+        auto reserve = [&](int which, unsigned n, unsigned long long* reserved, uint64_t* buf, unsigned long long cap) {
+            WarpAppender ap = app[which];
+            const unsigned long long pos = ap.reserve(n, reserved, buf, cap);
+            __syncwarp();
+            if (lane_id() == 0) app[which] = ap;
+            __syncwarp();
+            return pos;
+        };
+        if (ta) {
+            put(amask, a.acc, reserve(0, ta, &a.ctr->acc_reserved, a.acc, a.acc_cap) + (pre & 0xFFFFu), a.acc_cap);
+            n_screen_acc += __popc(amask);
+        }
+        if (tb)
+            put(bmask, a.band, reserve(1, tb, &a.ctr->band_reserved, a.band, a.band_cap) + (pre >> 16), a.band_cap);
+    }
+    cp_async_wait<0>();
+    WarpAppender app_acc = app[0], app_band = app[1];
     app_acc.pad(a.acc, a.acc_cap);
     app_band.pad(a.band, a.band_cap);
 #pragma unroll
@@ -168,8 +345,8 @@ __global__ void __launch_bounds__(kPT, 1) plain_kernel(const PlainArgs a) {
     if (lane_id() == 0) {
         if (app_acc.valid) atomicAdd(&a.ctr->acc_valid, app_acc.valid);
         if (app_band.valid) atomicAdd(&a.ctr->band_valid, app_band.valid);
-        if (n_screen_acc) atomicAdd(&a.ctr->screen_accept, n_screen_acc);
-        if (threadIdx.x == 0 && n_items) atomicAdd(&a.ctr->items, n_items);
+        if (n_screen_acc) atomicAdd(&a.ctr->screen_accept, (unsigned long long)n_screen_acc);
+        if (threadIdx.x == 0 && n_items) atomicAdd(&a.ctr->items, (unsigned long long)n_items);
     }
 }
 
@@ -424,11 +601,13 @@ void screen_plain(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) 
         a.cls[c].r_emit = R.emit;
         a.cls[c].s_emit = S.emit;
         a.cls[c].d = R.d;
+        a.cls[c].vec = R.d % 4 == 0 ? 1 : 0;   // the prepared sides are 256-byte aligned
     }
     DBuf<float2> dth((size_t)g.njoins, st);
     fp32_sum_thresholds(g, dth.p, st);
-    a.chunks = g.cand->chunks.p;
-    a.nchunks = g.cand->dev_counts.p + 1;
+    a.off = g.cand->off.p;
+    a.total = g.cand->dev_counts.p;
+    a.ntR = g.ntR_total;
     a.jlist = g.cand->jlist.p;
     a.rtiles = g.rtiles;
     a.stiles = g.stiles;
