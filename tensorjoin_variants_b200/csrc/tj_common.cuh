@@ -41,15 +41,15 @@ struct Counters {
     unsigned long long items;          // tile pairs screened
     unsigned long long band_fp64;      // band pairs that reached the FP64 terminal
     unsigned long long xl_items;       // int8 four-product screen: items that took the low-limb products
+    unsigned long long longest_row;    // most pairs of one row (canonical output by rows)
     unsigned long long status;         // kStatus* bits
     unsigned long long pairs_screened; // distance evaluations of the candidate list
     unsigned long long screen_ops;     // algorithmic screen operations of the candidate list
     unsigned long long class_items[4]; // candidate tile pairs per class
     unsigned long long screen_reserved;  // acc_reserved after the screen, before the refinement appends
     unsigned long long chunk_next;       // work queue of the one-SM screen: chunks taken beyond the first wave
-    unsigned long long pad[1];
 };
-constexpr int kCountersPerAttempt = 10;
+constexpr int kCountersPerAttempt = 11;
 
 // Per-join parameters (batched mode has one per join; a single join uses one entry).
 struct JoinParams {

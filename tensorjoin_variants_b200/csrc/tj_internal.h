@@ -102,8 +102,9 @@ void stage_reset();
 
 // ------------------------------------------------------------------ scan / sort (tj_sort.cu)
 size_t scan_workspace_elems(size_t n);
+// with `longest` (device, u64) the largest element is raised into it
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
-                        cudaStream_t st);
+                        cudaStream_t st, unsigned long long* longest = nullptr);
 size_t radix_workspace_elems(size_t n);
 void radix_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp, size_t n, int bits,
                 uint32_t* ws, cudaStream_t st, unsigned long long* status = nullptr, bool* in_tmp = nullptr);
@@ -305,6 +306,38 @@ void decode_pairs_batched(const uint64_t* keys, long long n, const unsigned long
                           const long long* n_cols, int njoins, int64_t* i_out, int64_t* j_out, cudaStream_t st);
 void batch_offsets(const uint64_t* keys, long long n, const unsigned long long* key_off, int njoins,
                    long long* offsets, cudaStream_t st);
+
+// ------------------------------------------------------------------ canonical output by rows (tj_output.cu)
+// Key space and rows of one join: key = key_off + i * n_cols + j, its rows numbered from row_off.
+struct RowTable {
+    unsigned long long key_off, row_off, n_cols, recip;   // recip = floor((2^64 - 1) / n_cols)
+};
+struct RowTables {
+    int njoins = 1;
+    RowTable first{};                                  // the only join's table
+    const RowTable* tab = nullptr;                     // device, batches
+    const unsigned long long* key_off = nullptr;       // device, batches: key_off and row_off of each join
+    const unsigned long long* row_off = nullptr;
+};
+RowTable make_row_table(unsigned long long key_off, unsigned long long row_off, unsigned long long n_cols);
+constexpr unsigned long long kLongRow = 16384;         // longest row order_rows sorts
+// Counts the pairs of every row (device slot count, at most cap) and scans the counts: first[r] is row
+// r's first position; *longest is raised to the largest count.  cnt and first may be one array.
+void count_rows(const uint64_t* keys, const Counters* ctr, unsigned long long cap, const RowTables& t, bool directed,
+                uint32_t nrows, uint32_t* cnt, uint32_t* first, unsigned long long* longest, uint32_t* ws,
+                cudaStream_t st);
+// Puts the columns of the keys in canonical order; `cursor` (first positions) ends as the rows' ends.
+void order_rows(const uint64_t* keys, unsigned long long slots, const RowTables& t, bool directed, uint32_t nrows,
+                uint32_t total, unsigned long long longest, uint32_t* cursor, uint32_t* cols,
+                unsigned long long* status, cudaStream_t st);
+void rows_pairs(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, const RowTables& t, int64_t* i_out,
+                int64_t* j_out, cudaStream_t st);
+void rows_keys(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, const RowTables& t, uint64_t* out,
+               cudaStream_t st);
+void rows_neighbors(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, uint32_t* counts, int64_t* flat,
+                    cudaStream_t st);
+void rows_batch_offsets(const uint32_t* row_end, const unsigned long long* row_off, int njoins, long long n,
+                        long long* out, cudaStream_t st);
 
 int num_sms();
 // limit of the screen kernels' pipeline waits for joins started on the calling thread (tj_set_wait_limit)

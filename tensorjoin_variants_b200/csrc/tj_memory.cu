@@ -93,7 +93,7 @@ struct Cached {
     size_t cap;
     cudaEvent_t ev;   // recorded on the releasing stream when the buffer was given back
 };
-constexpr size_t kCacheEntries = 4;
+constexpr size_t kCacheEntries = 6;   // a join's accept buffer, rows and columns, and a held result's
 constexpr size_t kCacheBytes = (size_t)32 << 30;
 std::mutex g_cache_mu;
 std::vector<Cached> g_cache[kMaxDev];

@@ -21,78 +21,106 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr size_t kScanOne = 4 * kScanTile;   // up to here one block scans everything
 
-// Block-wide exclusive scan of kScanTile u32 values; writes block totals.
-__global__ void __launch_bounds__(kScanThreads) scan_tiles(const uint32_t* in, uint32_t* out, size_t n,
-                                                           uint32_t* sums) {
-    __shared__ uint32_t warp_tot[32];
-    const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
+TJ_DEV uint32_t load_items(const uint32_t* in, size_t base, size_t n, uint32_t (&v)[kScanItems], uint32_t& most) {
     uint32_t local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         v[k] = (base + k < n) ? in[base + k] : 0u;
         local += v[k];
+        most = max(most, v[k]);
     }
-    unsigned tot;
+    return local;
+}
+// Exclusive scan of one value per thread over the block; `all` gets the block's total.
+TJ_DEV uint32_t block_scan(uint32_t local, uint32_t* warp_tot, uint32_t& all) {
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned pre = warp_excl_scan(local, tot);
+    unsigned tot;
+    const unsigned pre = warp_excl_scan(local, tot);
+    __syncthreads();   // the previous use of warp_tot is over
     if (lane == 0) warp_tot[warp] = tot;
     __syncthreads();
-    if (warp == 0) {
-        unsigned wt = warp_tot[lane], all;
-        unsigned wp = warp_excl_scan(wt, all);
-        warp_tot[lane] = wp;
-        if (lane == 0 && sums) sums[blockIdx.x] = all;
-    }
-    __syncthreads();
-    uint32_t run = pre + warp_tot[warp];
+    unsigned every;
+    const unsigned before = warp_excl_scan(warp_tot[lane], every);
+    all = every;
+    return pre + __shfl_sync(0xffffffffu, before, warp);
+}
+TJ_DEV void store_items(uint32_t* out, size_t base, size_t n, uint32_t run, const uint32_t (&v)[kScanItems]) {
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < n) out[base + k] = run;
         run += v[k];
     }
 }
-
-__global__ void add_block_offsets(uint32_t* out, size_t n, const uint32_t* offs) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += offs[i / kScanTile];
+TJ_DEV void raise_longest(unsigned long long* longest, uint32_t most) {
+    if (!longest) return;
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane_id() == 0 && most) atomicMax(longest, (unsigned long long)most);
 }
 
-__global__ void write_total(const uint32_t* in_last, const uint32_t* out_last, uint32_t* total) {
-    *total = *in_last + *out_last;
+// Short arrays: one block, tile after tile.
+__global__ void __launch_bounds__(kScanThreads) scan_one(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total,
+                                                         unsigned long long* longest) {
+    __shared__ uint32_t warp_tot[32];
+    uint32_t carry = 0, most = 0;
+    for (size_t t = 0; t < n; t += kScanTile) {
+        const size_t base = t + (size_t)threadIdx.x * kScanItems;
+        uint32_t v[kScanItems], all;
+        const uint32_t local = load_items(in, base, n, v, most);
+        const uint32_t pre = block_scan(local, warp_tot, all);
+        store_items(out, base, n, carry + pre, v);
+        carry += all;
+    }
+    if (total && threadIdx.x == 0) *total = carry;
+    raise_longest(longest, most);
+}
+
+// Longer arrays: the tiles' sums, then every tile adds up the sums before it and scans itself.
+__global__ void __launch_bounds__(kScanThreads) scan_sums(const uint32_t* in, size_t n, uint32_t* sums,
+                                                          unsigned long long* longest) {
+    __shared__ uint32_t warp_tot[32];
+    uint32_t v[kScanItems], most = 0, all;
+    const uint32_t local =
+        load_items(in, (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems, n, v, most);
+    block_scan(local, warp_tot, all);
+    if (threadIdx.x == 0) sums[blockIdx.x] = all;
+    raise_longest(longest, most);
+}
+__global__ void __launch_bounds__(kScanThreads) scan_apply(const uint32_t* in, uint32_t* out, size_t n,
+                                                           const uint32_t* sums, uint32_t* total) {
+    __shared__ uint32_t warp_tot[32];
+    uint32_t part = 0, before, all, v[kScanItems], most = 0;
+    for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads) part += sums[b];
+    block_scan(part, warp_tot, before);
+    const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
+    const uint32_t local = load_items(in, base, n, v, most);
+    const uint32_t pre = block_scan(local, warp_tot, all);
+    store_items(out, base, n, before + pre, v);
+    if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + all;
 }
 
 }  // namespace
 
-size_t scan_workspace_elems(size_t n) {
-    size_t total = 0;
-    while (n > 1) {
-        n = (n + kScanTile - 1) / kScanTile;
-        total += n + 1;
-    }
-    return total + 1;
-}
+size_t scan_workspace_elems(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
 // out[i] = sum_{k<i} in[k]; optional *total = sum of all (device pointer).
-// `ws` needs scan_workspace_elems(n) u32 elements.  `in` and `out` may alias.
+// `ws` needs scan_workspace_elems(n) u32 elements.  `in` and `out` may alias.  One launch up to 16,384
+// elements, two above (the recursive form it replaces took three to six, and small joins are bound by
+// the number of launches).
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
-                        cudaStream_t st) {
+                        cudaStream_t st, unsigned long long* longest) {
     if (n == 0) {
-        if (total) cudaMemsetAsync(total, 0, sizeof(uint32_t), st);
+        if (total) TJ_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), st));
         return;
     }
-    const size_t nb = (n + kScanTile - 1) / kScanTile;
-    // keep a copy of the last input element when aliasing in/out, for the total
-    uint32_t* last_copy = ws;  // 1 element
-    uint32_t* sums = ws + 1;
-    if (total) cudaMemcpyAsync(last_copy, in + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-    launch(scan_tiles, (unsigned)nb, kScanThreads, 0, st, in, out, n, nb > 1 ? sums : nullptr);
-    if (nb > 1) {
-        exclusive_scan_u32(sums, sums, nb, nullptr, sums + nb, st);
-        launch(add_block_offsets, (unsigned)((n + 255) / 256), 256, 0, st, out, n, sums);
+    if (n <= kScanOne) {
+        launch(scan_one, 1, kScanThreads, 0, st, in, out, n, total, longest);
+        return;
     }
-    if (total) launch(write_total, 1, 1, 0, st, last_copy, out + (n - 1), total);
+    const unsigned nb = (unsigned)((n + kScanTile - 1) / kScanTile);
+    launch(scan_sums, nb, kScanThreads, 0, st, in, n, ws, longest);
+    launch(scan_apply, nb, kScanThreads, 0, st, in, out, n, (const uint32_t*)ws, total);
 }
 
 // ------------------------------------------------------------------ radix sort
