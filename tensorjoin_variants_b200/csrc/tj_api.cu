@@ -139,16 +139,23 @@ __global__ void cell_starts(const uint32_t* flag, const uint32_t* pos, long long
 // pairs per class (out[2 + c] = class_items[c], for the issued-operation count).
 __global__ void pairs_screened_kernel(const uint4* chunks, const uint32_t* nchunks, const uint32_t* jlist,
                                       const uint4* rtiles, const uint4* stiles, const ScreenOps ops, int half,
-                                      unsigned long long* out) {
+                                      int group, unsigned long long* out) {
     unsigned long long acc = 0, aops = 0, items[kMaxClass] = {0, 0, 0, 0};
     const unsigned n = *nchunks;
     for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         const uint4 ch = chunks[c];
-        const uint4 rt = rtiles[ch.x];
+        const uint4 rt = rtiles[ch.x * group];
         const unsigned long long rv = rt.y;
         unsigned long long p = 0, hi = 0;   // hi: 128-column half-items issued
         for (unsigned e = ch.y; e < ch.z; ++e) {
             const uint32_t je = jlist[e];
+            if (group > 1) {   // lists of R tile groups, the live tiles in the top bits
+                const unsigned m = je >> (32 - group), nv = stiles[je & ((1u << (32 - group)) - 1u)].y;
+                for (int k = 0; k < group; ++k)
+                    if ((m >> k) & 1u) p += (unsigned long long)rtiles[ch.x * group + k].y * nv;
+                hi += 2 * __popc(m);
+                continue;
+            }
             const unsigned nv = stiles[je & kJMask].y;
             if (!half) {
                 p += rv * nv;
@@ -349,7 +356,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
             fail(TJ_ERR_INVALID, "the int8-limb screen needs an integer eps2 below 2^62");
         total_r += j.nR;
     }
-    const int chunk_items = (opt && opt->chunk_items > 0) ? opt->chunk_items : 64;
+    int chunk_items = (opt && opt->chunk_items > 0) ? opt->chunk_items : 64;
     const int esize = dtype == TJ_DTYPE_I16 ? 2 : 4;
     tj_stats& S_ = res->stats;
     memset(&S_, 0, sizeof(S_));
@@ -524,6 +531,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         // the screen packs half-tiles)
         TileSet* halves = half_packed ? &K.tSh : nullptr;
         K.R.src = srcR; K.R.dtype = dtype; K.R.n = roR[njc]; K.R.d = d; K.R.screen = screen;
+        K.R.i8_four = i8 && ((opt && (opt->flags & TJ_FLAG_I8_FOUR_PRODUCTS)) || d > kI8HighLimbPad);
         K.R.njc = njc; K.R.d_rowoff = njc > 1 ? K.rowoffR.p : nullptr;
         if (self)
             prepare_side(K.R, K.fp.p, K.pca_frame, K.center.p, st, &ctr.p->status, &K.tS, stile, halves);
@@ -533,6 +541,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         Side* pS = &K.R;
         if (!self) {
             K.S.src = srcS; K.S.dtype = dtype; K.S.n = roS[njc]; K.S.d = d; K.S.screen = screen;
+            K.S.i8_four = K.R.i8_four;
             K.S.njc = njc; K.S.d_rowoff = njc > 1 ? K.rowoffS.p : nullptr;
             prepare_side(K.S, K.fp.p, K.pca_frame, K.center.p, st, &ctr.p->status, &K.tS, stile, halves);
             compute_perm_local(K.S, st);
@@ -610,9 +619,15 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     ev.rec(1, st);
 
     // candidate tile pairs (block-diagonal over joins) and execution chunks
+    // the int8 high-limb screen takes R tiles in groups, and chunks short enough that every SM gets several
+    const int rgroup = i8 && i8_high_limb_screen(g) ? i8_rtiles(C[0]->R.kpad / 128) : 1;
+    if (rgroup > 1 && !(opt && opt->chunk_items > 0)) {
+        const long long lists = (g.ntR_total + rgroup - 1) / rgroup, entries = lists * g.ntS_total / (self ? 2 : 1);
+        chunk_items = (int)std::min(64ll, std::max(4ll, entries / (num_sms() * 6) / 2 * 2));
+    }
     Candidates cand;
     if (nj == 1) {
-        build_candidates(*g.tR[0], *g.tS[0], jps[0].Tp, self, chunk_items, cand, st);
+        build_candidates(*g.tR[0], *g.tS[0], jps[0].Tp, self, chunk_items, cand, st, rgroup);
     } else {
         std::vector<CandClassView> views(ncls);
         for (int c = 0; c < ncls; ++c) {
@@ -656,9 +671,9 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         sops.per_pair[c] = (unsigned long long)cls_d[c] * (i8 ? 8ull : (C[c]->R.split ? 6ull : 2ull));
         // one half-item issues 2 M N K per product: 128 x 128 (16-bit, 3 products with the split; a
         // tile pair is two half-items) or 128 x 128 x 1/2 (int8: an item is one 128 x 128 tile pair,
-        // counted as two halves, of which the high-limb screen issues hh only)
-        sops.per_item[c] = 2.0 * kTileR * 128.0 * (double)C[c]->R.kpad * (C[c]->R.split ? 3.0 : 1.0) *
-                           (i8 ? 0.5 : 1.0);
+        // counted as two halves, of which the high-limb screen issues hh and the folded norms only)
+        sops.per_item[c] = 2.0 * kTileR * 128.0 * (double)(C[c]->R.kpad + (i8 && !C[c]->R.i8_four ? kI8Fold : 0)) *
+                           (C[c]->R.split ? 3.0 : 1.0) * (i8 ? 0.5 : 1.0);
     }
     g.half_packed = half_packed;
     if (g.half_packed) {
@@ -683,7 +698,8 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     }
     launch(pairs_screened_kernel, num_sms() * 4, 256, 0, st, (const uint4*)cand.chunks.p,
            (const uint32_t*)(cand.dev_counts.p + 1), (const uint32_t*)cand.jlist.p, (const uint4*)d_rt.p,
-           (const uint4*)d_st.p, sops, g.half_packed ? 1 : 0, &ctr.p->pairs_screened);
+           (const uint4*)d_st.p, sops, g.half_packed ? 1 : 0, rgroup,
+           &ctr.p->pairs_screened);
     ev.rec(6, st);
 
     // optional screen-error sampling (tensor-core screens): 64 tile pairs spread over the candidate list

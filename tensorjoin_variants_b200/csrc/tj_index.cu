@@ -607,7 +607,7 @@ template <int kScreen, int kSplit, int kL>   // kL lanes per row (4, 8 or 32): 3
 __global__ void prep_rows(const void* src, int dtype, long long n, int d, int kpad, long long rows_pad,
                           const uint32_t* perm, const float* center, uint16_t* op, int8_t* op8, float* xs,
                           double* nrm2, float* nrm2f, float* zn, float* en, float* yn, float* zl, long long* inorm,
-                          unsigned long long* status) {
+                          int8_t* foldR, int8_t* foldS, I8Row* rec, unsigned long long* status) {
     const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kL;
     const unsigned sub = threadIdx.x % kL;
     const bool live = r < rows_pad;          // lanes past the end still take part in the shuffles
@@ -699,6 +699,26 @@ __global__ void prep_rows(const void* src, int dtype, long long n, int d, int kp
         nrm2[r] = sx;
         nrm2f[r] = __double2float_rn(sx);
         if (inorm) inorm[r] = sq;
+    }
+    if (kScreen == kScreenInt8Limb && rec) {
+        const int base = (int)((threadIdx.x & 31u) & ~(unsigned)(kL - 1));
+        const double hn = __shfl_sync(0xffffffffu, rt, base + 1), ln = __shfl_sync(0xffffffffu, rt, base + 3);
+        // 1 / sqrt(128), rounded up with room for the rounding of the product
+        constexpr double kInv = 0.08838834764831845 * (1.0 + 0x1p-40);
+        const int H = real ? (int)ceil(hn * kInv) : 0, L = real ? (int)ceil(ln * kInv) : 0;
+        const int G = real ? (int)ceil((hn + ln * 0x1p-7) * kInv) : 0;
+        const int b = real ? (int)min(sq >> 15, (long long)kI8FoldMax) : kI8FoldMax;   // no point: the least value
+        const int s = b / 127, each = s / kI8FoldDigits, more = s % kI8FoldDigits;
+        if (live)
+            for (int k = sub; k < kI8Fold; k += kL) {
+                const int digit = k < kI8FoldDigits ? -(each + (k < more ? 1 : 0)) : -(b % 127);
+                foldR[(size_t)r * kI8Fold + k] =
+                    (int8_t)(k < kI8FoldDigits ? 127 : k == kI8FoldDigits ? 1 : k == kI8FoldDigits + 1 ? H : L);
+                foldS[(size_t)r * kI8Fold + k] =
+                    (int8_t)(k <= kI8FoldDigits ? digit : k == kI8FoldDigits + 1 ? L : G);
+            }
+        if (live && sub == 0)
+            rec[r] = I8Row{real ? sq : 0ll, (uint32_t)orig, (uint8_t)H, (uint8_t)L, (uint8_t)G, 0};
     }
 }
 
@@ -1592,34 +1612,48 @@ __global__ void __launch_bounds__(256) cand_test_batched(const CandBlock* blocks
     }
 }
 
-__global__ void cand_count(const uint32_t* bitmap, int words, int ntR, uint32_t* cnt) {
+// With `step` > 1 a list is that of `step` consecutive R tiles (the S tiles that are a candidate for any
+// of them), and the top `step` bits of its entries say for which.
+TJ_DEV uint32_t any_of(const uint32_t* rows, int words, int w, int n) {
+    uint32_t b = 0;
+    for (int k = 0; k < n; ++k) b |= rows[(size_t)k * words + w];
+    return b;
+}
+__global__ void cand_count(const uint32_t* bitmap, int words, int ntR, int step, uint32_t* cnt) {
     const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
-    if (I >= ntR) return;
+    if (I * step >= ntR) return;
+    const uint32_t* rows = bitmap + (size_t)I * step * words;
+    const int n = min(step, ntR - I * step);
     unsigned c = 0;
-    for (int w = lane; w < words; w += 32) c += __popc(bitmap[(size_t)I * words + w]);
+    for (int w = lane; w < words; w += 32) c += __popc(any_of(rows, words, w, n));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if (lane == 0) cnt[I] = c;
 }
 
-__global__ void cand_fill(const uint32_t* bitmap, int words, int ntR, const uint32_t* off, uint32_t* jlist,
+__global__ void cand_fill(const uint32_t* bitmap, int words, int ntR, int step, const uint32_t* off, uint32_t* jlist,
                           const uint32_t* rtile_sbase) {
     const int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned lane = threadIdx.x & 31;
-    if (I >= ntR) return;
+    if (I * step >= ntR) return;
+    const uint32_t* rows = bitmap + (size_t)I * step * words;
+    const int n = min(step, ntR - I * step);
     uint32_t pos = off[I];
     const uint32_t sb = rtile_sbase ? rtile_sbase[I] : 0u;   // batched: global id of the join's first S tile
     for (int w0 = 0; w0 < words; w0 += 32) {
         const int w = w0 + lane;
-        const unsigned bits = w < words ? bitmap[(size_t)I * words + w] : 0u;
+        const unsigned bits = w < words ? any_of(rows, words, w, n) : 0u;
         unsigned tot;
         const unsigned pre = warp_excl_scan(__popc(bits), tot);
         unsigned b = bits, p = pos + pre;
         while (b) {
             const int bit = __ffs(b) - 1;
             b &= b - 1;
-            jlist[p++] = sb + (uint32_t)(w * 32 + bit);
+            uint32_t j = sb + (uint32_t)(w * 32 + bit);
+            if (step > 1)
+                for (int k = 0; k < n; ++k) j |= ((rows[(size_t)k * words + w] >> bit) & 1u) << (32 - step + k);
+            jlist[p++] = j;
         }
         pos += tot;
     }
@@ -1958,9 +1992,9 @@ void prepare_side(Side& s, const FrameParams* fpd, bool pca_frame, const float* 
             std::swap(s.keys, ktmp);
             std::swap(s.perm, vtmp);
         }
-        // joins on int14 rows (one join, 128-row tiles): rows inside each tile by norm (the sorted
-        // keys are not read again on this path)
-        if (i8 && ts && tile == 128 && s.njc <= 1)
+        // the four-product screen of int14 rows tests groups of 8 columns against their least norm: rows
+        // inside each 128-row tile by norm (the sorted keys are not read again on this path)
+        if (s.i8_four && ts && tile == 128 && s.njc <= 1)
             launch(order_tile_rows_by_norm, (unsigned)((n + 127) / 128), 128, 0, st, s.src, s.dtype, n, s.d,
                    s.perm.p);
     }
@@ -1971,6 +2005,11 @@ void prepare_side(Side& s, const FrameParams* fpd, bool pca_frame, const float* 
     if (i8) {
         s.op8 = DBuf<int8_t>(rp * 2 * s.kpad, st);
         s.inorm = DBuf<long long>(rp, st);
+        if (!s.i8_four) {
+            s.foldR = DBuf<int8_t>(rp * kI8Fold, st);
+            s.foldS = DBuf<int8_t>(rp * kI8Fold, st);
+            s.rec = DBuf<I8Row>(rp, st);
+        }
     }
     if (s.screen == kScreenPlain) s.xs = DBuf<float>(rp * s.d, st);
     s.nrm2 = DBuf<double>(rp, st);
@@ -1987,7 +2026,7 @@ void prepare_side(Side& s, const FrameParams* fpd, bool pca_frame, const float* 
 #define TJ_PREP_L(SCR, SPLIT, L)                                                                                 \
     launch(prep_rows<SCR, SPLIT, L>, (unsigned)((rp * L + 255) / 256), 256, 0, st, s.src, s.dtype, n, s.d, s.kpad, \
            s.rows_pad, s.perm.p, center, s.op.p, s.op8.p, s.xs.p, s.nrm2.p, s.nrm2f.p, s.zn.p, s.en.p, s.yn.p,      \
-           s.zl.p, s.inorm.p, status)
+           s.zl.p, s.inorm.p, s.foldR.p, s.foldS.p, s.rec.p, status)
 #define TJ_PREP(SCR, SPLIT)                                    \
     do {                                                       \
         if (s.kpad <= 16) TJ_PREP_L(SCR, SPLIT, 4);            \
@@ -2058,9 +2097,10 @@ void compute_perm_local(Side& s, cudaStream_t st) {
 }
 
 void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self_join, int chunk_items,
-                      Candidates& c, cudaStream_t st) {
-    const int ntR = tr.ntiles, ntS = ts.ntiles, d = tr.d;
+                      Candidates& c, cudaStream_t st, int group) {
+    const int ntiles = tr.ntiles, ntS = ts.ntiles, d = tr.d;
     const int words = (ntS + 31) / 32;
+    const int step = group, ntR = (ntiles + step - 1) / step;   // ntR: lists
     c.cnt = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.off = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.dev_counts = DBuf<uint32_t>(2, st);
@@ -2070,24 +2110,24 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
     c.chunks_cap = maxc / (size_t)chunk_items + (size_t)ntR + 1;
     c.chunks = DBuf<uint4>(c.chunks_cap, st);
     if (ntR == 0 || ntS == 0) return;
-    DBuf<uint32_t> bitmap((size_t)ntR * words, st);
+    DBuf<uint32_t> bitmap((size_t)ntiles * words, st);
     TJ_CUDA(cudaMemsetAsync(bitmap.p, 0, bitmap.bytes(), st));
     const int ci = (size_t)3 * 16 * d * sizeof(float) <= 200 * 1024 ? 16 : (size_t)3 * 4 * d * sizeof(float) <= 200 * 1024 ? 4 : 1;
     const size_t smem = (size_t)3 * ci * d * sizeof(float);
     if (smem > 200 * 1024) fail(-7, "dimension too large for the candidate test");
-    dim3 grid((unsigned)((ntS + 255) / 256), (unsigned)((ntR + ci - 1) / ci));
+    dim3 grid((unsigned)((ntS + 255) / 256), (unsigned)((ntiles + ci - 1) / ci));
 #define TJ_CAND(CI)                                                                                                 \
     TJ_CUDA(cudaFuncSetAttribute(cand_test<CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
-    launch(cand_test<CI>, grid, 256, smem, st, tr.ctrT.p, tr.loT.p, tr.hiT.p, tr.rad.p, ntR, ts.ctrT.p, ts.loT.p,      \
+    launch(cand_test<CI>, grid, 256, smem, st, tr.ctrT.p, tr.loT.p, tr.hiT.p, tr.rad.p, ntiles, ts.ctrT.p, ts.loT.p,      \
                                            ts.hiT.p, ts.rad.p, ntS, d, tr.tile, ts.tile, Tp, self_join ? 1 : 0,      \
                                            bitmap.p, words)
     if (ci == 16) { TJ_CAND(16); } else if (ci == 4) { TJ_CAND(4); } else { TJ_CAND(1); }
 #undef TJ_CAND
     TJ_CUDA(cudaGetLastError());
-    launch(cand_count, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, c.cnt.p);
+    launch(cand_count, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntiles, step, c.cnt.p);
     DBuf<uint32_t> sws(scan_workspace_elems((size_t)ntR) + 4, st);
     exclusive_scan_u32(c.cnt.p, c.off.p, (size_t)ntR, c.dev_counts.p, sws.p, st);
-    launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, c.off.p, c.jlist.p,
+    launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntiles, step, c.off.p, c.jlist.p,
            (const uint32_t*)nullptr);
     // chunks: (w, I) order so that concurrently running CTAs share the same S window
     DBuf<uint32_t> nch((size_t)ntR, st), cbase((size_t)ntR, st);
@@ -2165,10 +2205,10 @@ void build_candidates_batched(const std::vector<CandClassView>& classes, const s
     TJ_CUDA(cudaFuncSetAttribute(cand_test_batched<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch(cand_test_batched<16>, nb, 256, smem, st, (const CandBlock*)dblk.p, (const CandClassView*)dview.p,
            (const double*)dtp.p, bitmap.p, words);
-    launch(cand_count, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, c.cnt.p);
+    launch(cand_count, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, 1, c.cnt.p);
     DBuf<uint32_t> sws(scan_workspace_elems((size_t)ntR) + 4, st);
     exclusive_scan_u32(c.cnt.p, c.off.p, (size_t)ntR, c.dev_counts.p, sws.p, st);
-    launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, c.off.p, c.jlist.p,
+    launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, 1, c.off.p, c.jlist.p,
            (const uint32_t*)dsb.p);
     DBuf<uint32_t> nch((size_t)ntR, st), cbase((size_t)ntR, st);
     launch(chunk_counts, (unsigned)((ntR + 255) / 256), 256, 0, st, c.cnt.p, ntR, chunk_items, nch.p);

@@ -117,6 +117,24 @@ enum DType { kF32 = 0, kI16 = 1 };
 enum Mode { kModeRS = 0, kModeUpper = 1, kModeDirected = 2 };
 enum Screen { kScreenPlain = 0, kScreenBF16 = 1, kScreenFP16 = 2, kScreenInt8Limb = 3, kScreenBF16X3 = 4, kScreenFP16X3 = 5 };
 
+// ------------------------------------------------------------------ int8 high-limb screen: folded rows
+// Rows of up to kI8HighLimbPad padded elements.  32 more int8 elements per row and side:
+//   R side: 127 (kI8FoldDigits times), 1, H, L;   S side: digits of -b, all in [-128, 0], L, G
+// whose product is H_i L_j + L_i G_j - b_j, with b = floor(|q|^2 / 2^15), folded as at most kI8FoldMax
+// (an |q|^2 of 1.5 10^10, 230 elements of the largest size; a smaller b only lets more pairs through),
+// and the limb norms in units of sqrt(128), rounded up: H >= |h|, L >= |l|, G >= |h| + |l| / 128.
+constexpr int kI8HighLimbPad = 256;
+constexpr int kI8Fold = 32, kI8FoldDigits = kI8Fold - 3;
+constexpr int kI8FoldMax = 127 * 128 * kI8FoldDigits + 126;
+struct I8Row {           // what a candidate pair needs of a row
+    long long norm;      // exact |q|^2
+    uint32_t id;         // emitted row id
+    uint8_t H, L, G, pad;
+};
+static_assert(sizeof(I8Row) == 16, "a tile's records are one bulk copy");
+// R tiles a CTA of the high-limb screen holds, by k-blocks of 128 elements (shared memory)
+__host__ __device__ constexpr int i8_rtiles(int kblocks) { return kblocks == 1 ? 4 : 2; }
+
 // ------------------------------------------------------------------ prepared side (tj_index.cu)
 // A side of the join in Morton order: permutation, MMA operand and per-row certificate metadata.
 // Row r of every array is the point perm[r] of the caller's input.
@@ -145,6 +163,9 @@ struct Side {
     DBuf<float> yn;              // [rows_pad] upper bound of ||x - centre||
     DBuf<float> zl;              // [rows_pad] upper bound of ||z_lo|| (0 without the split)
     DBuf<long long> inorm;       // [rows_pad] exact integer squared norms (int path)
+    bool i8_four = false;        // int8 limbs: prepared for the four-product screen
+    DBuf<int8_t> foldR, foldS;   // [rows_pad, kI8Fold] folded elements as the R and as the S side (high-limb screen)
+    DBuf<I8Row> rec;             // [rows_pad] row records (high-limb screen)
 };
 
 // Tile statistics at one tile granularity (128 rows for R, 256 rows for S).
@@ -204,8 +225,10 @@ bool compute_frame(const void* const* srcs, const long long* ns, int nsrc, int d
 void prepare_side(Side& s, const FrameParams* fp_dev, bool pca_frame, const float* center, cudaStream_t st,
                   unsigned long long* status, TileSet* ts = nullptr, int tile = 0, TileSet* halves = nullptr);
 void tile_stats(const Side& s, int tile, TileSet& ts, cudaStream_t st);
+// With `group` > 1 the lists are those of groups of consecutive R tiles, and the top `group` bits of a
+// list entry say which of them it is for (the int8 high-limb screen).
 void build_candidates(const TileSet& tr, const TileSet& ts, double T, bool self_join, int chunk_items,
-                      Candidates& c, cudaStream_t st);
+                      Candidates& c, cudaStream_t st, int group = 1);
 void gather_rows(const std::vector<const void*>& srcs, const std::vector<long long>& rows, int d, int esize,
                  void* dst, cudaStream_t st);
 void compute_perm_local(Side& s, cudaStream_t st);
