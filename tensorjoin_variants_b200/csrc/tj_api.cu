@@ -211,11 +211,24 @@ int bits_for(unsigned long long max_value) {
     return b;
 }
 
+// The calling thread's events on the current device, made once (creating and destroying eight per join
+// cost a small join more than its kernels; joins of one thread run one after the other).
 struct Events {
-    cudaEvent_t e[8];
+    struct Set {
+        cudaEvent_t e[8] = {};
+        ~Set() { for (auto& x : e) if (x) cudaEventDestroy(x); }
+    };
+    cudaEvent_t* e;
     int n = 0;
-    Events() { for (auto& x : e) cudaEventCreate(&x); }
-    ~Events() { for (auto& x : e) cudaEventDestroy(x); }
+    Events() {
+        static thread_local Set sets[64];
+        int dev = 0;
+        TJ_CUDA(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64) fail(TJ_ERR_INVALID, "device ordinal out of range");
+        e = sets[dev].e;
+        for (int i = 0; i < 8; ++i)
+            if (!e[i]) TJ_CUDA(cudaEventCreate(&e[i]));
+    }
     void rec(int i, cudaStream_t st) { cudaEventRecord(e[i], st); n = i + 1 > n ? i + 1 : n; }
     double ms(int a, int b) const {
         float m = 0.f;
@@ -333,6 +346,20 @@ void check_flags(const tj_options* opt) {
     if (opt->stages != 0 && (opt->stages < 2 || opt->stages > 6)) fail(TJ_ERR_INVALID, "stages must be 0 or 2..6");
 }
 
+// Joins that are done directly, without an index: no options (every knob is one of the indexed path) and
+// rows of at most 192 elements (longer ones belong to the CTA-pair screen).  The direct path takes 75 us
+// plus about 0.1 ps per pair and element (8 more elements per pair for its classification); the indexed
+// path's forty launches and two waits take 350 to 700 us however small the join.  The line lies at 2^31,
+// 300 us, below the smallest figure measured for the indexed path on the same joins (one B200, whole
+// call, direct | indexed): 311 x 256 x 8 80 | 419 us; 5,003 x 3,217 x 65 214 | 584; 10,000 x 2 directed 184 |
+// 421; 8,000 x 16 upper 154 | 448; 8,000 x 8,000 x 32 291 | 654; beyond it 20,000 x 2 directed 508 | 454.
+bool direct_join_fits(const JoinIn& j, int mode, const tj_options* opt) {
+    if (opt && (opt->initial_capacity || opt->chunk_items || opt->flags || opt->k_block || opt->stages)) return false;
+    const long long nS = mode == TJ_MODE_RS ? j.nS : j.nR;
+    if (j.d > 192 || j.nR < 1 || nS < 1 || j.nR > (1ll << 15) || nS > (1ll << 20)) return false;
+    return (double)j.nR * (double)nS / (mode == TJ_MODE_UPPER ? 2 : 1) * (j.d + 8) <= 0x1p31;
+}
+
 // One or many joins.  Joins are grouped into classes of equal d; each class gets one
 // concatenated, Morton-sorted side per operand (joins stay contiguous), global tile tables, one
 // block-diagonal candidate list and one persistent screen launch over all classes.
@@ -402,6 +429,37 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     stage_reset();
     Events ev;
     ev.rec(0, st);
+    if (nj == 1 && !i8 && direct_join_fits(joins[0], mode, opt)) {
+        // A small join: all pairs at once, without an index.  Elements beyond what every screen takes (FP16
+        // operands: 65504 after centring, so 30000 before) go through the screen that was asked for, which
+        // accepts or refuses them.
+        const JoinIn& j = joins[0];
+        const JoinParams jp = make_params(j.eps2, j.d, 64, 0, j.nR, ncols[0], self);
+        const bool half = screen == TJ_SCREEN_FP16 || screen == TJ_SCREEN_FP16X3;
+        unsigned long long hdr[5];
+        const bool upper = mode == TJ_MODE_UPPER;
+        if (join_direct((const float*)j.R, (unsigned)j.nR, (const float*)(self ? j.R : j.S), (unsigned)ncols[0], upper,
+                        jp, half ? 30000.f : 0x1p40f, res->rows, res->cols, hdr, st, ev.e[1], ev.e[2])) {
+            ev.rec(3, st);
+            TJ_CUDA(cudaStreamSynchronize(st));
+            res->n_all_rows = (uint32_t)j.nR;
+            res->tabs.first = make_row_table(0, 0, (unsigned long long)ncols[0]);
+            res->count = (long long)hdr[0];
+            // counts as of a screen over all tile pairs; a directed join's are those of its i < j pairs
+            const long long sym = mode == TJ_MODE_DIRECTED ? 2 : 1, own = mode == TJ_MODE_DIRECTED ? j.nR : 0;
+            S_.tile_pairs = ((j.nR + kTileR - 1) / kTileR) * ((ncols[0] + kTileS - 1) / kTileS);
+            S_.pairs_screened = S_.pairs_all;
+            S_.band = S_.band_fp64 = S_.rare_checks = (int64_t)hdr[3] / sym;
+            S_.refine_accept = (int64_t)hdr[4] / sym;
+            S_.screen_accept = (res->count - own) / sym - S_.refine_accept;
+            S_.result_pairs = res->count;
+            S_.screen_ops = S_.screen_ops_issued = 2.0 * j.d * (double)S_.pairs_screened;
+            S_.ms_screen = ev.ms(1, 2);
+            S_.ms_sort = ev.ms(2, 3);
+            S_.ms_total = ev.ms(0, 3);
+            return;
+        }
+    }
     DBuf<Counters> ctr(1, st);
     launch(zero_counters, 1, 32, 0, st, ctr.p, 0);
 

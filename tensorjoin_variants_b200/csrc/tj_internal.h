@@ -319,6 +319,13 @@ void screen_i8(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st);
 // true when screen_i8 runs the high-limb screen (hh products only; undecided pairs go to the band
 // and the exact integer refinement), false for the four-product screen (exact, no band)
 bool i8_high_limb_screen(const ScreenInput& g);
+// One small join in full, without an index: FP32 direct differences of all pairs, FP64 for the few that
+// they leave open, the accepted pairs as a bitmap and from it the rows' ends and columns.  False (and
+// nothing made) when an element is not a number within `limit`.  hdr: pairs, longest row, (that flag),
+// pairs decided in FP64 and accepted there.  The events are recorded around the distances.
+bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool upper, const JoinParams& jp, float limit,
+                 DBuf<uint32_t>& rows, DBuf<uint32_t>& cols, unsigned long long (&hdr)[5], cudaStream_t st,
+                 cudaEvent_t screen0, cudaEvent_t screen1);
 // FP64 terminal for the band; fp32_stage puts the certified FP32 band stage in front of it.
 void refine_band(const ScreenInput& g, const EmitBuffers& eb, bool fp32_stage, cudaStream_t st);
 void expand_directed(const uint64_t* upper, unsigned long long n_upper_slots, uint64_t* out, long long N,

@@ -14,6 +14,7 @@
 // the same FP64 refinement of band pairs.  It plays the role of the reference's
 // GDS-Join FP64 grid join / FP32-first control (adapters/gds_g2a/kernel.cu:314-386,
 // g15_strong_control_20260905/src/fp32_first.py:104-157).
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -23,6 +24,29 @@
 namespace tj {
 
 namespace {
+
+// Squared distance in the oracle's order: sequential k, one FP64 rounding per operation.
+TJ_DEV double seq_d2(const float* x, const float* y, int d) {
+    double acc = 0.0;
+    if ((d & 3) == 0 && ((((uintptr_t)x) | ((uintptr_t)y)) & 15) == 0) {
+        const float4* x4 = (const float4*)x;
+        const float4* y4 = (const float4*)y;
+        for (int k = 0; k < d / 4; ++k) {
+            const float4 a = __ldg(x4 + k), b = __ldg(y4 + k);
+            double t;
+            t = __dsub_rn((double)a.x, (double)b.x); acc = __dadd_rn(acc, __dmul_rn(t, t));
+            t = __dsub_rn((double)a.y, (double)b.y); acc = __dadd_rn(acc, __dmul_rn(t, t));
+            t = __dsub_rn((double)a.z, (double)b.z); acc = __dadd_rn(acc, __dmul_rn(t, t));
+            t = __dsub_rn((double)a.w, (double)b.w); acc = __dadd_rn(acc, __dmul_rn(t, t));
+        }
+    } else {
+        for (int k = 0; k < d; ++k) {
+            const double t = __dsub_rn((double)__ldg(x + k), (double)__ldg(y + k));
+            acc = __dadd_rn(acc, __dmul_rn(t, t));
+        }
+    }
+    return acc;
+}
 
 // ------------------------------------------------------------------ plain FP32 join
 // A unit is 128 R rows x 64 S rows (a quarter of a candidate tile pair); a CTA of 16 x 16 threads
@@ -56,7 +80,21 @@ struct PlainClass {
     int vec;             // rows are multiples of 16 bytes, 16-byte aligned
 };
 
+// Direct joins (kDirect below): every pair of one small join, straight from the caller's rows.
+struct DirectArgs {
+    unsigned nR, nS;            // rows
+    unsigned cols64;            // units per R tile: ceil(nS / 64)
+    int upper;                  // 1: self-join, columns above the row only
+    int diagonal;               // 1: self-join with self pairs (always accepted, not counted as decided)
+    unsigned long long* bits;   // [nR][cols64] accepted pairs, bit c of word u: column 64 u + c
+    uint32_t* cnt;              // [nR] accepted pairs per row (zeroed)
+    unsigned long long* band;   // [2] pairs decided in FP64, and those of them accepted (zeroed)
+    double T;
+    float2 thr;
+};
+
 struct PlainArgs {
+    DirectArgs dir;
     const uint32_t* off;        // [ntR] first candidate of each R tile
     const uint32_t* total;      // candidates
     int ntR;
@@ -112,17 +150,24 @@ TJ_DEV int find_rtile(const uint32_t* off, int n, uint32_t e) {
     return lo;
 }
 
+// kDirect: the units are all quarters of the join's own grid, taken in turn by the CTAs; a unit's
+// accepted pairs go to a bitmap instead of the emit buffers, and the few pairs the FP32 sum cannot decide
+// are decided by the thread that finds them, in FP64 from the rows.
+template <bool kDirect>
 __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
     __shared__ __align__(16) float sm[kPStages][kPRows][kPLd];
     __shared__ PlainStage info[kPStages];
     __shared__ uint32_t ids[kPStages][kPRows];   // emitted row ids of the unit's rows and columns
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     // this CTA's run of all candidates' quarters, in candidate order: candidate e, quarter p, `left` units
-    const unsigned long long units = (unsigned long long)*a.total * kPUnits;
+    // (direct: e is the unit, left counts this CTA's)
+    const unsigned long long units = kDirect ? (unsigned long long)((a.dir.nR + kTileR - 1) / kTileR) * a.dir.cols64
+                                             : (unsigned long long)*a.total * kPUnits;
     const unsigned long long u0 = units * blockIdx.x / gridDim.x;
-    unsigned left = (unsigned)(units * (blockIdx.x + 1) / gridDim.x - u0);
-    uint32_t e = (uint32_t)(u0 / kPUnits);
-    unsigned p = (unsigned)(u0 % kPUnits) * kPCols;
+    unsigned left = kDirect ? (unsigned)(units > blockIdx.x ? (units - 1 - blockIdx.x) / gridDim.x + 1 : 0)
+                            : (unsigned)(units * (blockIdx.x + 1) / gridDim.x - u0);
+    uint32_t e = kDirect ? blockIdx.x : (uint32_t)(u0 / kPUnits);
+    unsigned p = kDirect ? 0u : (unsigned)(u0 % kPUnits) * kPCols;
     __shared__ WarpAppender apps[kPT / 32][2];   // accept and band of each warp: touched by hits only
     WarpAppender* app = apps[threadIdx.x >> 5];
     if (lane_id() < 2) app[lane_id()] = WarpAppender();
@@ -138,7 +183,7 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
     // issued a quarter apart so that neither is waited for
     uint2 stt = make_uint2(0, 0), stn = stt;
     uint32_t jn = 0;
-    const uint32_t total = *a.total;
+    const uint32_t total = kDirect ? 0u : *a.total;
     bool self_join = false, first = true;
     float2 th = make_float2(0.f, 0.f);
     auto s_tile = [&](uint32_t j) { return *reinterpret_cast<const uint2*>(a.stiles + j); };
@@ -146,6 +191,10 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
     const unsigned lr = threadIdx.x >> 2, lq = (threadIdx.x & 3) * 4;
     auto step = [&] {
         --left;
+        if (kDirect) {
+            e += gridDim.x;
+            return;
+        }
         p += kPCols;
         if (p == (unsigned)kTileS) {
             p = 0;
@@ -155,7 +204,18 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
     };
     auto issue = [&](int buf) {
         // the unit's tiles (units without a column, or at or below a self-join's diagonal, are passed over)
-        while (k0 == 0 && left) {
+        while (kDirect && k0 == 0 && left) {
+            const unsigned I = e / a.dir.cols64, u = e - I * a.dir.cols64;
+            rt = make_uint4(I * kTileR, min((unsigned)kTileR, a.dir.nR - I * kTileR), 0u, 0u);
+            stt = make_uint2(u * kPCols, min((unsigned)kPCols, a.dir.nS - u * kPCols));
+            th = a.dir.thr;
+            const PlainClass& pc = a.cls[0];
+            pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.d + lq;
+            pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.d + lq;
+            if (!(a.dir.upper && stt.x + kPCols <= rt.x + 1)) break;   // (the bitmap of an upper join starts at 0)
+            step();
+        }
+        while (!kDirect && k0 == 0 && left) {
             if (fresh) {
                 fresh = false;
                 if (e >= e_end) {
@@ -210,7 +270,7 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         }
         if (threadIdx.x == 0)
             info[buf] = PlainStage{rt.x, rt.y, c0, nvJ, rt.z, kc, k0 == 0, k0 + kc >= d, th};
-        if (k0 + kc >= d && threadIdx.x < kPRows) {
+        if (!kDirect && k0 + kc >= d && threadIdx.x < kPRows) {
             const unsigned t = threadIdx.x;
             cp_async4_zfill(&ids[buf][t], t < kTileR ? pc.r_emit + rt.x + min(t, rt.y - 1)
                                                      : pc.s_emit + c0 + min(t - kTileR, nvJ - 1), true);
@@ -279,11 +339,13 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
 #pragma unroll
         for (int i = 0; i < kPI; ++i) rm[i] = fminf(fmin3(v[i * kPJ], v[i * kPJ + 1], v[i * kPJ + 2]), v[i * kPJ + 3]);
         const float m = fmin3(fmin3(rm[0], rm[1], rm[2]), fmin3(rm[3], rm[4], rm[5]), fminf(rm[6], rm[7]));
-        if (!__any_sync(0xffffffffu, !(m > in.th.y))) continue;
+        const bool near = __any_sync(0xffffffffu, !(m > in.th.y));
+        if (!kDirect && !near) continue;
+        unsigned long long word = 0;   // direct: columns accepted in row tx * 16 + ty (tx < 8)
         unsigned rows = 0;
 #pragma unroll
         for (int i = 0; i < kPI; ++i) rows |= rm[i] > in.th.y ? 0u : 1u << i;
-        rows = __reduce_or_sync(0xffffffffu, rows);
+        rows = near ? __reduce_or_sync(0xffffffffu, rows) : 0u;
         uint32_t cand = 0, amask = 0;
 #pragma unroll
         for (int i = 0; i < kPI; ++i) {
@@ -298,8 +360,8 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         const int ni = min(max((int)in.nvI - ty + 15, 0) >> 4, kPI), nj = min(max((int)in.nvJ - tx + 15, 0) >> 4, kPJ);
         const uint32_t rmask = ni == kPI ? 0xFFFFFFFFu : (1u << (kPJ * ni)) - 1u;
         cand &= rmask & (((1u << nj) - 1u) * 0x11111111u);
-        const JoinParams& jp = a.jps[in.join];
-        if (jp.self_join && in.c0 <= in.r0 + kTileR - 1) {   // keep sorted column > sorted row only
+        const bool above = kDirect ? a.dir.upper != 0 : a.jps[in.join].self_join != 0;
+        if (above && in.c0 <= in.r0 + kTileR - 1) {   // keep (sorted) column > (sorted) row only
             uint32_t w = cand;
             while (w) {
                 const int b = __ffs(w) - 1;
@@ -309,6 +371,44 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         }
         amask &= cand;
         const uint32_t bmask = cand & ~amask;
+        if (kDirect) {
+            if (near) {
+                uint32_t w = bmask;
+                while (w) {   // the oracle's own sum
+                    const int b = __ffs(w) - 1;
+                    w &= w - 1;
+                    const PlainClass& pc = a.cls[0];
+                    if (a.dir.diagonal && in.r0 + (b / kPJ) * 16 + ty == in.c0 + (b % kPJ) * 16 + tx) {
+                        amask |= 1u << b;
+                        continue;
+                    }
+                    const bool ok = seq_d2(pc.rx + (size_t)(in.r0 + (b / kPJ) * 16 + ty) * pc.d,
+                                           pc.sx + (size_t)(in.c0 + (b % kPJ) * 16 + tx) * pc.d, pc.d) <= a.dir.T;
+                    if (ok) amask |= 1u << b;
+                    atomicAdd(a.dir.band, 1ull);
+                    if (ok) atomicAdd(a.dir.band + 1, 1ull);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < kPI; ++i) {
+                    if (!(rows & (1u << i))) continue;
+                    unsigned long long wi = 0;
+#pragma unroll
+                    for (int j = 0; j < kPJ; ++j) {
+                        const unsigned bal = __ballot_sync(0xffffffffu, (amask >> (i * kPJ + j)) & 1u);
+                        wi |= (unsigned long long)((bal >> (threadIdx.x & 16)) & 0xFFFFu) << (16 * j);
+                    }
+                    word = tx == i ? wi : word;
+                }
+            }
+            const unsigned row = tx * 16 + ty;
+            if (tx < kPI && row < in.nvI) {
+                a.dir.bits[(size_t)(in.r0 + row) * a.dir.cols64 + in.c0 / kPCols] = word;
+                if (word) atomicAdd(a.dir.cnt + in.r0 + row, (unsigned)__popcll(word));
+            }
+            continue;
+        }
+        const JoinParams& jp = a.jps[in.join];
         unsigned tot;
         const unsigned pre = warp_excl_scan(__popc(amask) | (__popc(bmask) << 16), tot);
         const unsigned ta = tot & 0xFFFFu, tb = tot >> 16;
@@ -337,6 +437,7 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
             put(bmask, a.band, reserve(1, tb, &a.ctr->band_reserved, a.band, a.band_cap) + (pre >> 16), a.band_cap);
     }
     cp_async_wait<0>();
+    if (kDirect) return;
     WarpAppender app_acc = app[0], app_band = app[1];
     app_acc.pad(a.acc, a.acc_cap);
     app_band.pad(a.band, a.band_cap);
@@ -389,28 +490,6 @@ TJ_DEV float fp32_d2(const float* x, const float* y, int d) {
         }
     }
     return (a0 + a1) + (a2 + a3);
-}
-
-TJ_DEV double seq_d2(const float* x, const float* y, int d) {
-    double acc = 0.0;
-    if ((d & 3) == 0 && ((((uintptr_t)x) | ((uintptr_t)y)) & 15) == 0) {
-        const float4* x4 = (const float4*)x;
-        const float4* y4 = (const float4*)y;
-        for (int k = 0; k < d / 4; ++k) {
-            const float4 a = __ldg(x4 + k), b = __ldg(y4 + k);
-            double t;
-            t = __dsub_rn((double)a.x, (double)b.x); acc = __dadd_rn(acc, __dmul_rn(t, t));
-            t = __dsub_rn((double)a.y, (double)b.y); acc = __dadd_rn(acc, __dmul_rn(t, t));
-            t = __dsub_rn((double)a.z, (double)b.z); acc = __dadd_rn(acc, __dmul_rn(t, t));
-            t = __dsub_rn((double)a.w, (double)b.w); acc = __dadd_rn(acc, __dmul_rn(t, t));
-        }
-    } else {
-        for (int k = 0; k < d; ++k) {
-            const double t = __dsub_rn((double)__ldg(x + k), (double)__ldg(y + k));
-            acc = __dadd_rn(acc, __dmul_rn(t, t));
-        }
-    }
-    return acc;
 }
 
 // Exact squared distance of two int16 rows in int64: each difference fits int32 and its square
@@ -570,23 +649,145 @@ __global__ void batch_offsets_kernel(const uint64_t* keys, long long n, const un
 // summation tree of depth <= d + 2): s <= x certifies the FP64 oracle value <= T, s > y certifies
 // it > T.  |s - D| <= gamma_{d+4} D + (d + 4) 2^-147 with u = 2^-24 (one rounding in each
 // difference, one in each FMA or add along the tree, subnormal products absolutely).
+static float2 fp32_sum_threshold(const JoinParams& jp) {
+    const double u = 0x1p-24, nu = (double)(jp.d + 4) * u;
+    const double gam = nu / (1.0 - nu);
+    const double tiny = (double)(jp.d + 4) * 0x1p-147;
+    const double tin = (jp.Tm - tiny) * (1.0 - gam) * (1.0 - 0x1p-30);
+    const double tout = (jp.Tp + tiny) * (1.0 + gam) * (1.0 + 0x1p-30) + tiny;
+    float fin = tin > 0 ? (float)tin : -1.f;   // nearest, then nudged to stay a lower bound
+    if (fin > 0 && (double)fin > tin) fin = nextafterf(fin, 0.f);
+    float fout = (float)tout;
+    if ((double)fout < tout) fout = nextafterf(fout, INFINITY);
+    return make_float2(fin, fout);
+}
 static void fp32_sum_thresholds(const ScreenInput& g, float2* dst, cudaStream_t st) {
     const JoinParams* hj = g.h_jps;
     if (!hj) fail(-1, "the FP32 thresholds need the host join parameters");
     std::vector<float2> th((size_t)g.njoins);
-    for (int k = 0; k < g.njoins; ++k) {
-        const double u = 0x1p-24, nu = (double)(hj[k].d + 4) * u;
-        const double gam = nu / (1.0 - nu);
-        const double tiny = (double)(hj[k].d + 4) * 0x1p-147;
-        const double tin = (hj[k].Tm - tiny) * (1.0 - gam) * (1.0 - 0x1p-30);
-        const double tout = (hj[k].Tp + tiny) * (1.0 + gam) * (1.0 + 0x1p-30) + tiny;
-        float fin = tin > 0 ? (float)tin : -1.f;   // nearest, then nudged to stay a lower bound
-        if (fin > 0 && (double)fin > tin) fin = nextafterf(fin, 0.f);
-        float fout = (float)tout;
-        if ((double)fout < tout) fout = nextafterf(fout, INFINITY);
-        th[k] = make_float2(fin, fout);
-    }
+    for (int k = 0; k < g.njoins; ++k) th[k] = fp32_sum_threshold(hj[k]);
     upload(dst, th.data(), g.njoins * sizeof(float2), st);
+}
+
+namespace {
+
+// Direct joins, before the distances: every element within `limit` in magnitude (NaN and infinities are
+// not), and the row counts and band counters zeroed.  One flag per block, so that nothing needs to be
+// zeroed for this kernel itself.
+__global__ void __launch_bounds__(256) direct_check(const float* R, size_t nr, const float* S, size_t ns, float limit,
+                                                    uint32_t* cnt, unsigned nR, unsigned long long* band,
+                                                    uint32_t* bad) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool ok = true;
+    for (size_t i = t0; i < nr; i += stride) ok &= fabsf(R[i]) <= limit;
+    for (size_t i = t0; i < ns; i += stride) ok &= fabsf(S[i]) <= limit;
+    for (size_t i = t0; i < nR; i += stride) cnt[i] = 0;
+    if (t0 < 2) band[t0] = 0;
+    const int any = __syncthreads_or(!ok);
+    if (threadIdx.x == 0) bad[blockIdx.x] = any ? 1u : 0u;
+}
+
+// Exclusive scan of the row counts by one block, and what the host reads: pairs, longest row, whether an
+// element was out of range, and the band counters.
+__global__ void __launch_bounds__(1024) direct_scan(uint32_t* cnt, unsigned nR, const uint32_t* bad, unsigned nbad,
+                                                    const unsigned long long* band, unsigned long long* hdr) {
+    __shared__ unsigned wt[32];
+    unsigned flag = 0, longest = 0;
+    for (unsigned i = threadIdx.x; i < nbad; i += 1024) flag |= bad[i];
+    unsigned long long carry = 0;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    constexpr unsigned kEach = 8;   // consecutive rows per thread
+    for (unsigned t = 0; t < nR; t += 1024 * kEach) {
+        unsigned v[kEach], sum = 0;
+#pragma unroll
+        for (unsigned k = 0; k < kEach; ++k) {
+            const unsigned i = t + threadIdx.x * kEach + k;
+            v[k] = i < nR ? cnt[i] : 0u;
+            sum += v[k];
+            longest = max(longest, v[k]);
+        }
+        unsigned tot, all;
+        const unsigned pre = warp_excl_scan(sum, tot);
+        __syncthreads();
+        if (lane == 0) wt[warp] = tot;
+        __syncthreads();
+        const unsigned wpre = warp_excl_scan(wt[lane], all);
+        const unsigned before = __shfl_sync(0xffffffffu, wpre, warp);
+        unsigned run = (uint32_t)carry + before + pre;
+#pragma unroll
+        for (unsigned k = 0; k < kEach; ++k) {
+            const unsigned i = t + threadIdx.x * kEach + k;
+            run += v[k];
+            if (i < nR) cnt[i] = run;   // the row's end
+        }
+        carry += all;
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    __syncthreads();
+    if (lane == 0) wt[warp] = longest;
+    const int any = __syncthreads_or(flag != 0);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 32; ++w) longest = max(longest, wt[w]);
+        hdr[0] = carry;
+        hdr[1] = longest;
+        hdr[2] = any ? 1 : 0;
+        hdr[3] = band[0];
+        hdr[4] = band[1];
+    }
+}
+
+// Columns of every row in order, from the bitmap: a warp per row, 32 words at a time.
+__global__ void __launch_bounds__(256) direct_emit(const unsigned long long* bits, unsigned nR, unsigned cols64,
+                                                   const uint32_t* row_end, uint32_t* cols) {
+    const unsigned row = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = lane_id();
+    if (row >= nR) return;   // warp-uniform
+    uint32_t pos = row ? row_end[row - 1] : 0u;
+    const uint32_t end = row_end[row];
+    for (unsigned u0 = 0; u0 < cols64 && pos < end; u0 += 32) {
+        const unsigned u = u0 + lane;
+        unsigned long long w = u < cols64 ? bits[(size_t)row * cols64 + u] : 0ull;
+        unsigned tot;
+        uint32_t p = pos + warp_excl_scan((unsigned)__popcll(w), tot);
+        for (; w; w &= w - 1) cols[p++] = u * 64 + (unsigned)__ffsll((long long)w) - 1;
+        pos += tot;
+    }
+}
+
+}  // namespace
+
+bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool upper, const JoinParams& jp, float limit,
+                 DBuf<uint32_t>& rows, DBuf<uint32_t>& cols, unsigned long long (&hdr)[5], cudaStream_t st,
+                 cudaEvent_t screen0, cudaEvent_t screen1) {
+    const unsigned cols64 = (nS + kPCols - 1) / kPCols;
+    rows = DBuf<uint32_t>::result(nR, st);
+    DBuf<unsigned long long> bits((size_t)nR * cols64, st), band(2 + 5, st);
+    const size_t er = (size_t)nR * jp.d, es = R == S ? 0 : (size_t)nS * jp.d;
+    const unsigned nb = (unsigned)std::min<size_t>((size_t)num_sms() * 2, (er + es + nR + 1023) / 1024);
+    DBuf<uint32_t> bad(nb, st);
+    if (upper) TJ_CUDA(cudaMemsetAsync(bits.p, 0, bits.bytes(), st));   // units below the diagonal are passed over
+    launch(direct_check, nb, 256, 0, st, R, er, S, es, limit, rows.p, nR, band.p, bad.p);
+    PlainArgs a;
+    memset(&a, 0, sizeof(a));
+    a.cls[0] = PlainClass{R, S, nullptr, nullptr, jp.d,
+                          jp.d % 4 == 0 && ((((uintptr_t)R) | ((uintptr_t)S)) & 15) == 0 ? 1 : 0};
+    a.dir = DirectArgs{nR, nS, cols64, upper ? 1 : 0, R == S && !upper ? 1 : 0, bits.p, rows.p, band.p, jp.T, fp32_sum_threshold(jp)};
+    const unsigned units = (nR + kTileR - 1) / kTileR * cols64;
+    cudaEventRecord(screen0, st);
+    launch(plain_kernel<true>, std::min(units, (unsigned)num_sms() * 2), kPT, 0, st, a);
+    cudaEventRecord(screen1, st);
+    launch(direct_scan, 1, 1024, 0, st, rows.p, nR, (const uint32_t*)bad.p, nb, (const unsigned long long*)band.p,
+           band.p + 2);
+    TJ_CUDA(cudaMemcpyAsync(hdr, band.p + 2, sizeof(hdr), cudaMemcpyDeviceToHost, st));
+    TJ_CUDA(cudaStreamSynchronize(st));
+    if (hdr[2]) {
+        rows.reset();
+        return false;
+    }
+    cols = DBuf<uint32_t>::result(std::max<size_t>((size_t)hdr[0], 1), st);
+    if (hdr[0])
+        launch(direct_emit, (nR + 7) / 8, 256, 0, st, (const unsigned long long*)bits.p, nR, cols64,
+               (const uint32_t*)rows.p, cols.p);
+    return true;
 }
 
 void screen_plain(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) {
@@ -618,7 +819,7 @@ void screen_plain(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) 
     a.band = eb.band;
     a.band_cap = eb.band_cap;
     a.ctr = eb.ctr;
-    launch(plain_kernel, num_sms() * 2, kPT, 0, st, a);
+    launch(plain_kernel<false>, num_sms() * 2, kPT, 0, st, a);
 }
 
 void refine_band(const ScreenInput& g, const EmitBuffers& eb, bool fp32_stage, cudaStream_t st) {
