@@ -589,6 +589,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         // the screen packs half-tiles)
         TileSet* halves = half_packed ? &K.tSh : nullptr;
         K.R.src = srcR; K.R.dtype = dtype; K.R.n = roR[njc]; K.R.d = d; K.R.screen = screen;
+        for (int q = 0; q < njc; ++q) K.R.longest = std::max(K.R.longest, joins[J[q]].nR);
         K.R.i8_four = i8 && ((opt && (opt->flags & TJ_FLAG_I8_FOUR_PRODUCTS)) || d > kI8HighLimbPad);
         K.R.njc = njc; K.R.d_rowoff = njc > 1 ? K.rowoffR.p : nullptr;
         if (self)
@@ -599,6 +600,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         Side* pS = &K.R;
         if (!self) {
             K.S.src = srcS; K.S.dtype = dtype; K.S.n = roS[njc]; K.S.d = d; K.S.screen = screen;
+            for (int q = 0; q < njc; ++q) K.S.longest = std::max(K.S.longest, joins[J[q]].nS);
             K.S.i8_four = K.R.i8_four;
             K.S.njc = njc; K.S.d_rowoff = njc > 1 ? K.rowoffS.p : nullptr;
             prepare_side(K.S, K.fp.p, K.pca_frame, K.center.p, st, &ctr.p->status, &K.tS, stile, halves);
@@ -928,7 +930,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
             TJ_CUDA(cudaMemcpyAsync(res->stage[q].p, src[q], ns[q] * 8, cudaMemcpyDeviceToDevice, st));
             if (ns[q] > 1) {
                 DBuf<uint64_t> t(ns[q], st);
-                DBuf<uint32_t> w(radix_workspace_elems(ns[q]), st);
+                DBuf<uint32_t> w(sweep_workspace_elems(ns[q]), st);
                 radix_sort(res->stage[q].p, nullptr, t.p, nullptr, ns[q], 64, w.p, st, &ctr.p->status);
             }
         }
@@ -983,7 +985,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
             // and the two buffers change places instead of copying the keys back
             const bool swap = radix_result_in_tmp(slots, bits);
             DBuf<uint64_t> ktmp = swap ? DBuf<uint64_t>::result(slots + gs, st) : DBuf<uint64_t>(slots + gs, st);
-            DBuf<uint32_t> ws(radix_workspace_elems(slots), st);
+            DBuf<uint32_t> ws(sweep_workspace_elems(slots), st);
             if (guards) launch(guard_fill, 1, 256, 0, st, ktmp.p + slots);
             bool in_tmp = false;
             radix_sort(keys.p, nullptr, ktmp.p, nullptr, slots, bits, ws.p, st, &ctr.p->status, swap ? &in_tmp : nullptr);

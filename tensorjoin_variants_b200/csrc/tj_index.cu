@@ -1485,6 +1485,17 @@ __global__ void __launch_bounds__(256, 3) prep_tiles_warp_kernel(const float* __
     }
 }
 
+// Rows [n, rp) of a side's operand and row arrays (fewer than 256 rows) set to zero.
+__global__ void __launch_bounds__(256) zero_tail(uint16_t* op, int opw, double* nrm2, float* a, float* b, float* c,
+                                                 float* d, float* e, long long n, long long rp) {
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+    for (long long i = n * opw + t; i < rp * opw; i += step) op[i] = 0;
+    for (long long i = n + t; i < rp; i += step) {
+        nrm2[i] = 0.0;
+        a[i] = b[i] = c[i] = d[i] = e[i] = 0.f;
+    }
+}
+
 // Candidate test: thread = one S tile J, 16 R tiles per block (from shared memory).
 // Keeps (I, J) unless a rigorous lower bound on every pair distance exceeds sqrt(Tp).
 template <int kCandI>
@@ -1659,43 +1670,51 @@ __global__ void cand_fill(const uint32_t* bitmap, int words, int ntR, int step, 
     }
 }
 
-__global__ void chunk_counts(const uint32_t* cnt, int ntR, int ch, uint32_t* nch) {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
-    if (I < ntR) nch[I] = (cnt[I] + ch - 1) / ch;
-}
-
-// Emit one (w, I) sort key per chunk; unused capacity gets the max key.
-__global__ void chunk_keys(const uint32_t* nch, const uint32_t* cbase, int ntR, size_t cap, uint64_t* keys,
-                           uint32_t* vals) {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
-    if (I >= ntR) return;
-    const uint32_t b = cbase[I], c = nch[I];
-    for (uint32_t w = 0; w < c; ++w) {
-        if (b + w < cap) {
-            keys[b + w] = ((uint64_t)w << 32) | (uint32_t)I;
-            vals[b + w] = b + w;
+// Execution chunks: list I is cut into chunks of `ch` entries, and chunk w of every list comes before chunk
+// w + 1 of any, lists in order, so that CTAs running at the same time share a window of S tiles.  The
+// place of chunk (w, I) has a closed form, sum over all lists of min(chunks, w) plus the lists before I
+// that reach w, so one launch places them all (they were sorted by (w, I) in up to 24).  A block takes one
+// w and kPlaceLists lists.
+constexpr unsigned kPlaceLists = 8192;
+__global__ void __launch_bounds__(1024) place_chunks(const uint32_t* cnt, const uint32_t* off, int ntR, unsigned ch,
+                                                     uint4* chunks, uint32_t* total) {
+    __shared__ unsigned wt[32];
+    const unsigned w = blockIdx.x, I0 = blockIdx.y * kPlaceLists, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned before = 0, all = 0;
+    for (unsigned i = t; i < (unsigned)ntR; i += 1024) {
+        const unsigned n = (cnt[i] + ch - 1) / ch;
+        before += min(n, w) + (i < I0 && n > w ? 1u : 0u);
+        all += n;
+    }
+    const unsigned sum = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) wt[warp] = sum;
+    __syncthreads();
+    unsigned base = __reduce_add_sync(0xffffffffu, wt[lane]);
+    for (unsigned I1 = I0; I1 < min(I0 + kPlaceLists, (unsigned)ntR); I1 += 1024) {   // block-uniform
+        const unsigned I = I1 + t;
+        const unsigned mine = I < (unsigned)ntR ? cnt[I] : 0u;
+        const bool has = mine > w * ch;
+        const unsigned bal = __ballot_sync(0xffffffffu, has);
+        __syncthreads();
+        if (lane == 0) wt[warp] = __popc(bal);
+        __syncthreads();
+        unsigned tot;
+        const unsigned pre = warp_excl_scan(wt[lane], tot);
+        const unsigned rank = __shfl_sync(0xffffffffu, pre, warp) + __popc(bal & ((1u << lane) - 1u));
+        if (has) {
+            const unsigned b = off[I] + w * ch;
+            chunks[base + rank] = make_uint4(I, b, min(b + ch, off[I] + mine), 0);
         }
+        base += tot;
     }
-}
-
-__global__ void fill_keys_max(uint64_t* keys, uint32_t* vals, size_t from, size_t cap, const uint32_t* total) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x + from;
-    if (i < cap && i >= *total) {
-        keys[i] = ~0ull;
-        vals[i] = 0xFFFFFFFFu;
+    if (w == 0 && blockIdx.y == 0) {   // chunks in all
+        __syncthreads();
+        const unsigned s = __reduce_add_sync(0xffffffffu, all);
+        if (lane == 0) wt[warp] = s;
+        __syncthreads();
+        const unsigned sum_all = __reduce_add_sync(0xffffffffu, wt[lane]);
+        if (t == 0) *total = sum_all;
     }
-}
-
-__global__ void chunk_emit(const uint64_t* keys, size_t cap, const uint32_t* total, const uint32_t* cnt,
-                           const uint32_t* off, int ch, uint4* chunks) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap) return;
-    if (i >= *total) return;
-    const uint64_t k = keys[i];
-    const uint32_t I = (uint32_t)(k & 0xFFFFFFFFu), w = (uint32_t)(k >> 32);
-    const uint32_t b = off[I] + w * (uint32_t)ch;
-    const uint32_t e = min(b + (uint32_t)ch, off[I] + cnt[I]);
-    chunks[i] = make_uint4(I, b, e, 0);
 }
 
 // Half-tile masks for the one-SM tensor-core screen.  A candidate (R tile I, S tile J) of 128 x 256
@@ -1910,13 +1929,9 @@ void prep_tiles(Side& s, const float* center, int tile, TileSet& ts, TileSet* ha
     ts.built = true;
     // rows past the last tile (the operand padding up to rows_pad) are zero
     const long long n = s.n, rp = s.rows_pad;
-    if (rp > n) {
-        const size_t opw = (size_t)s.kpad * (s.split ? 2 : 1);
-        TJ_CUDA(cudaMemsetAsync(s.op.p + (size_t)n * opw, 0, (size_t)(rp - n) * opw * sizeof(uint16_t), st));
-        TJ_CUDA(cudaMemsetAsync(s.nrm2.p + n, 0, (size_t)(rp - n) * sizeof(double), st));
-        float* fl[5] = {s.nrm2f.p, s.zn.p, s.en.p, s.yn.p, s.zl.p};
-        for (float* f : fl) TJ_CUDA(cudaMemsetAsync(f + n, 0, (size_t)(rp - n) * sizeof(float), st));
-    }
+    if (rp > n)
+        launch(zero_tail, 16, 256, 0, st, s.op.p, s.kpad * (s.split ? 2 : 1), s.nrm2.p, s.nrm2f.p, s.zn.p, s.en.p,
+               s.yn.p, s.zl.p, n, rp);
     if (ntiles == 0) return;
     const uint32_t* r0 = tabled ? (const uint32_t*)ts.row0.p : nullptr;
     const uint32_t* nvv = tabled ? (const uint32_t*)ts.nvalid.p : nullptr;
@@ -1975,22 +1990,29 @@ void prepare_side(Side& s, const FrameParams* fpd, bool pca_frame, const float* 
     s.perm = DBuf<uint32_t>((size_t)std::max<long long>(n, 1), st);
     s.keys = DBuf<uint64_t>((size_t)std::max<long long>(n, 1), st);
     if (n > 0) {
-        DBuf<uint64_t> ktmp((size_t)n, st);
-        DBuf<uint32_t> vtmp((size_t)n, st);
-        DBuf<uint32_t> ws(radix_workspace_elems((size_t)n), st);
         if (pca_frame)
             launch(morton_keys_pca, (unsigned)((n + 255) / 256), 256, 0, st, s.src, s.dtype, n, s.d, fpd, s.keys.p,
                    s.perm.p, s.d_rowoff, s.njc, center);
         else
             launch(morton_keys, (unsigned)((n + 255) / 256), 256, 0, st, s.src, s.dtype, n, s.d, fpd, s.keys.p,
                    s.perm.p, s.d_rowoff, s.njc);
-        int jbits = 0;
-        while ((1 << jbits) < s.njc) ++jbits;
-        bool in_tmp = false;
-        radix_sort(s.keys.p, s.perm.p, ktmp.p, vtmp.p, (size_t)n, 32 + jbits, ws.p, st, status, &in_tmp);
-        if (in_tmp) {   // odd number of passes: the sorted arrays are the temporaries
-            std::swap(s.keys, ktmp);
-            std::swap(s.perm, vtmp);
+        // small joins: each join's rows in one block; larger ones: radix passes over the whole side
+        const long long longest = s.longest ? s.longest : n;
+        if (longest <= kSegmentSort) {
+            if (s.njc > 1) s.perm_local = DBuf<uint32_t>((size_t)n, st);
+            segment_sort(s.keys.p, s.perm.p, s.perm_local.p, s.d_rowoff, s.njc, n, longest, st);
+        } else {
+            DBuf<uint64_t> ktmp((size_t)n, st);
+            DBuf<uint32_t> vtmp((size_t)n, st);
+            DBuf<uint32_t> ws(sweep_workspace_elems((size_t)n), st);
+            int jbits = 0;
+            while ((1 << jbits) < s.njc) ++jbits;
+            bool in_tmp = false;
+            radix_sort(s.keys.p, s.perm.p, ktmp.p, vtmp.p, (size_t)n, 32 + jbits, ws.p, st, status, &in_tmp);
+            if (in_tmp) {   // odd number of passes: the sorted arrays are the temporaries
+                std::swap(s.keys, ktmp);
+                std::swap(s.perm, vtmp);
+            }
         }
         // the four-product screen of int14 rows tests groups of 8 columns against their least norm: rows
         // inside each 128-row tile by norm (the sorted keys are not read again on this path)
@@ -2090,9 +2112,11 @@ void compute_perm_local(Side& s, cudaStream_t st) {
         s.emit = s.perm.p;
         return;
     }
-    s.perm_local = DBuf<uint32_t>((size_t)s.n, st);
-    launch(perm_local_kernel, (unsigned)((s.n + 255) / 256), 256, 0, st, s.keys.p, s.perm.p, s.d_rowoff, s.n,
-           s.perm_local.p);
+    if (!s.perm_local.p) {
+        s.perm_local = DBuf<uint32_t>((size_t)s.n, st);
+        launch(perm_local_kernel, (unsigned)((s.n + 255) / 256), 256, 0, st, s.keys.p, s.perm.p, s.d_rowoff, s.n,
+               s.perm_local.p);
+    }
     s.emit = s.perm_local.p;
 }
 
@@ -2104,14 +2128,15 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
     c.cnt = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.off = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.dev_counts = DBuf<uint32_t>(2, st);
-    TJ_CUDA(cudaMemsetAsync(c.dev_counts.p, 0, 2 * sizeof(uint32_t), st));
     const size_t maxc = (size_t)ntR * (size_t)ntS;
     c.jlist = DBuf<uint32_t>(std::max<size_t>(maxc, 1), st);
     c.chunks_cap = maxc / (size_t)chunk_items + (size_t)ntR + 1;
     c.chunks = DBuf<uint4>(c.chunks_cap, st);
-    if (ntR == 0 || ntS == 0) return;
-    DBuf<uint32_t> bitmap((size_t)ntiles * words, st);
-    TJ_CUDA(cudaMemsetAsync(bitmap.p, 0, bitmap.bytes(), st));
+    if (ntR == 0 || ntS == 0) {
+        TJ_CUDA(cudaMemsetAsync(c.dev_counts.p, 0, 2 * sizeof(uint32_t), st));
+        return;
+    }
+    DBuf<uint32_t> bitmap((size_t)ntiles * words, st);   // every word is written by the test
     const int ci = (size_t)3 * 16 * d * sizeof(float) <= 200 * 1024 ? 16 : (size_t)3 * 4 * d * sizeof(float) <= 200 * 1024 ? 4 : 1;
     const size_t smem = (size_t)3 * ci * d * sizeof(float);
     if (smem > 200 * 1024) fail(-7, "dimension too large for the candidate test");
@@ -2129,19 +2154,9 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
     exclusive_scan_u32(c.cnt.p, c.off.p, (size_t)ntR, c.dev_counts.p, sws.p, st);
     launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntiles, step, c.off.p, c.jlist.p,
            (const uint32_t*)nullptr);
-    // chunks: (w, I) order so that concurrently running CTAs share the same S window
-    DBuf<uint32_t> nch((size_t)ntR, st), cbase((size_t)ntR, st);
-    launch(chunk_counts, (unsigned)((ntR + 255) / 256), 256, 0, st, c.cnt.p, ntR, chunk_items, nch.p);
-    exclusive_scan_u32(nch.p, cbase.p, (size_t)ntR, c.dev_counts.p + 1, sws.p, st);
-    const size_t cap = c.chunks_cap;
-    DBuf<uint64_t> keys(cap, st), ktmp(cap, st);
-    DBuf<uint32_t> vals(cap, st), vtmp(cap, st);
-    launch(fill_keys_max, (unsigned)((cap + 255) / 256), 256, 0, st, keys.p, vals.p, 0, cap, c.dev_counts.p + 1);
-    launch(chunk_keys, (unsigned)((ntR + 255) / 256), 256, 0, st, nch.p, cbase.p, ntR, cap, keys.p, vals.p);
-    DBuf<uint32_t> rws(radix_workspace_elems(cap), st);
-    radix_sort(keys.p, vals.p, ktmp.p, vtmp.p, cap, 48, rws.p, st);
-    launch(chunk_emit, (unsigned)((cap + 255) / 256), 256, 0, st, keys.p, cap, c.dev_counts.p + 1, c.cnt.p, c.off.p,
-                                                               chunk_items, c.chunks.p);
+    launch(place_chunks, dim3((unsigned)((ntS + chunk_items - 1) / chunk_items), (unsigned)((ntR + kPlaceLists - 1) / kPlaceLists)), 1024,
+           0, st, (const uint32_t*)c.cnt.p, (const uint32_t*)c.off.p, ntR, (unsigned)chunk_items, c.chunks.p,
+           c.dev_counts.p + 1);
     TJ_CUDA(cudaGetLastError());
 }
 
@@ -2181,13 +2196,18 @@ void build_candidates_batched(const std::vector<CandClassView>& classes, const s
     c.cnt = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.off = DBuf<uint32_t>((size_t)std::max(ntR, 1), st);
     c.dev_counts = DBuf<uint32_t>(2, st);
-    TJ_CUDA(cudaMemsetAsync(c.dev_counts.p, 0, 2 * sizeof(uint32_t), st));
-    size_t maxc = 0;
-    for (const auto& b : blocks) maxc += (size_t)b.ni * b.nj;
+    size_t maxc = 0, most = 1;   // candidates at most, and of one R tile
+    for (const auto& b : blocks) {
+        maxc += (size_t)b.ni * b.nj;
+        most = std::max(most, (size_t)b.nj);
+    }
     c.jlist = DBuf<uint32_t>(std::max<size_t>(maxc, 1), st);
     c.chunks_cap = maxc / (size_t)chunk_items + (size_t)ntR + 1;
     c.chunks = DBuf<uint4>(c.chunks_cap, st);
-    if (ntR == 0 || nb == 0) return;
+    if (ntR == 0 || nb == 0) {
+        TJ_CUDA(cudaMemsetAsync(c.dev_counts.p, 0, 2 * sizeof(uint32_t), st));
+        return;
+    }
     int dmax = 1;
     for (const auto& v : classes) dmax = std::max(dmax, v.d);
     DBuf<CandBlock> dblk((size_t)nb, st);
@@ -2210,19 +2230,9 @@ void build_candidates_batched(const std::vector<CandClassView>& classes, const s
     exclusive_scan_u32(c.cnt.p, c.off.p, (size_t)ntR, c.dev_counts.p, sws.p, st);
     launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntR, 1, c.off.p, c.jlist.p,
            (const uint32_t*)dsb.p);
-    DBuf<uint32_t> nch((size_t)ntR, st), cbase((size_t)ntR, st);
-    launch(chunk_counts, (unsigned)((ntR + 255) / 256), 256, 0, st, c.cnt.p, ntR, chunk_items, nch.p);
-    exclusive_scan_u32(nch.p, cbase.p, (size_t)ntR, c.dev_counts.p + 1, sws.p, st);
-    const size_t cap = c.chunks_cap;
-    DBuf<uint64_t> keys(cap, st), ktmp(cap, st);
-    DBuf<uint32_t> vals(cap, st), vtmp(cap, st);
-    launch(fill_keys_max, (unsigned)((cap + 255) / 256), 256, 0, st, keys.p, vals.p, (size_t)0, cap,
-           (const uint32_t*)(c.dev_counts.p + 1));
-    launch(chunk_keys, (unsigned)((ntR + 255) / 256), 256, 0, st, nch.p, cbase.p, ntR, cap, keys.p, vals.p);
-    DBuf<uint32_t> rws(radix_workspace_elems(cap), st);
-    radix_sort(keys.p, vals.p, ktmp.p, vtmp.p, cap, 48, rws.p, st);
-    launch(chunk_emit, (unsigned)((cap + 255) / 256), 256, 0, st, keys.p, cap, (const uint32_t*)(c.dev_counts.p + 1),
-           c.cnt.p, c.off.p, chunk_items, c.chunks.p);
+    launch(place_chunks, dim3((unsigned)((most + chunk_items - 1) / chunk_items), (unsigned)((ntR + kPlaceLists - 1) / kPlaceLists)), 1024,
+           0, st, (const uint32_t*)c.cnt.p, (const uint32_t*)c.off.p, ntR, (unsigned)chunk_items, c.chunks.p,
+           c.dev_counts.p + 1);
 }
 
 }  // namespace tj

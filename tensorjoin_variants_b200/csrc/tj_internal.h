@@ -105,7 +105,14 @@ size_t scan_workspace_elems(size_t n);
 // with `longest` (device, u64) the largest element is raised into it
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
                         cudaStream_t st, unsigned long long* longest = nullptr);
-size_t radix_workspace_elems(size_t n);
+size_t radix_workspace_elems(size_t n);   // without a status word
+size_t sweep_workspace_elems(size_t n);   // with one
+// Sorts each segment [off[k], off[k + 1]) (off null: [0, n)) of at most kSegmentSort keys by the low 32
+// bits of its keys, stably; perm gets the positions the keys came from, and local (may be null) the same
+// within the segment.
+constexpr long long kSegmentSort = 8192;
+void segment_sort(uint64_t* keys, uint32_t* perm, uint32_t* local, const long long* off, int nseg, long long n,
+                  long long longest, cudaStream_t st);
 void radix_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp, size_t n, int bits,
                 uint32_t* ws, cudaStream_t st, unsigned long long* status = nullptr, bool* in_tmp = nullptr);
 int radix_passes(int bits);
@@ -152,6 +159,7 @@ struct Side {
     const uint32_t* emit = nullptr;   // ids written into pair keys: perm (one join) or perm_local
     const long long* d_rowoff = nullptr;   // device [njc + 1]: first source row of each join (batched)
     int njc = 1;                 // joins concatenated in this side
+    long long longest = 0;       // rows of the largest of them (0: n)
     DBuf<uint64_t> keys;         // [n] Morton keys (sorted)
     DBuf<uint16_t> op;           // [rows_pad, kpad or 2*kpad] bf16 / fp16 operand of x - centre
     DBuf<int8_t> op8;            // [rows_pad, 2*kpad] int8 limbs [hi | lo] (int8 limb screen)

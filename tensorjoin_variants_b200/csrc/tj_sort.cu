@@ -208,13 +208,10 @@ TJ_DEV uint32_t block_excl_scan(uint32_t v, uint32_t* warp_tot) {
 // ballots), the block's keys are regrouped by digit in shared memory, and then written
 // out in that order, so consecutive threads store consecutive addresses of one digit's run
 // (about 16 keys = 128 B per digit and tile for 8-bit digits) instead of scattered 8-byte words.
-template <bool kVals>
-__global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const uint64_t* keys_in, const uint32_t* vals_in,
-                                                        uint64_t* keys_out, uint32_t* vals_out, size_t n, int shift,
+__global__ void __launch_bounds__(kScThreads, 3) rs_scatter(const uint64_t* keys_in, uint64_t* keys_out, size_t n, int shift,
                                                         const uint32_t* offs, unsigned nblocks) {
     extern __shared__ __align__(16) unsigned char rs_dyn[];
     uint64_t* sk = (uint64_t*)rs_dyn;                      // [kRsTile] keys grouped by digit
-    uint32_t* sv = (uint32_t*)(rs_dyn + kRsTile * 8);      // [kRsTile] values (kVals)
     __shared__ uint32_t wcnt[kScWarps][256];   // per warp and digit: count, then tile-local start
     __shared__ uint32_t gdelta[256];   // global start minus tile-local start of each digit's run (mod 2^32)
     __shared__ uint32_t wtot[kScWarps];
@@ -227,7 +224,6 @@ __global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const ui
     const size_t tbase = (size_t)blockIdx.x * kRsTile;
     const size_t wbase = tbase + (size_t)warp * (kScRounds * 32);
     uint64_t k[kScRounds];
-    uint32_t v[kScRounds];
     uint32_t rank[kScRounds];
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
@@ -246,13 +242,6 @@ __global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const ui
         __syncwarp();
         if (ok && (peers & lt) == 0) wcnt[warp][dg] = prev + __popc(peers);
         __syncwarp();
-    }
-    if (kVals) {   // values load while the block meets at the barrier (fewer live registers above)
-#pragma unroll
-        for (int r = 0; r < kScRounds; ++r) {
-            const size_t i = wbase + (size_t)r * 32 + lane;
-            v[r] = i < n ? vals_in[i] : 0u;
-        }
     }
     __syncthreads();
     {   // per digit (threads 0..255): total over warps, tile-local start by a block scan, then each
@@ -281,7 +270,6 @@ __global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const ui
         if (rank[r] != 0xFFFFFFFFu) {
             const unsigned p = wcnt[warp][digit_of(k[r], shift)] + rank[r];
             sk[p] = k[r];
-            if (kVals) sv[p] = v[r];
         }
     }
     __syncthreads();
@@ -290,7 +278,6 @@ __global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const ui
         const uint64_t key = sk[p];
         const size_t pos = (size_t)(uint32_t)(gdelta[digit_of(key, shift)] + p);
         keys_out[pos] = key;
-        if (kVals) vals_out[pos] = sv[p];
     }
 }
 
@@ -302,16 +289,13 @@ __global__ void __launch_bounds__(kScThreads, kVals ? 2 : 3) rs_scatter(const ui
 // One launch replaces the four to five launches per pass of the multi-block path.
 constexpr unsigned kSmallSort = 16384;
 
-template <bool kVals>
-__global__ void __launch_bounds__(kScThreads) rs_small(uint64_t* keys, uint32_t* vals, uint64_t* ktmp,
-                                                      uint32_t* vtmp, unsigned n, int passes) {
+__global__ void __launch_bounds__(kScThreads) rs_small(uint64_t* keys, uint64_t* ktmp, unsigned n, int passes) {
     __shared__ uint32_t wcnt[kScWarps][256];
     __shared__ uint32_t base[256];     // this pass: next output position of each digit
     __shared__ uint32_t wtot[kScWarps];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
     const unsigned lt = (1u << lane) - 1u;
     uint64_t *kin = keys, *kout = ktmp;
-    uint32_t *vin = vals, *vout = vtmp;
     for (int pass = 0; pass < passes; ++pass) {
         const int shift = 8 * pass;
         if (t < 256) base[t] = 0;
@@ -363,19 +347,16 @@ __global__ void __launch_bounds__(kScThreads) rs_small(uint64_t* keys, uint32_t*
                     const unsigned i = wbase + r * 32 + lane;
                     const unsigned pos = wcnt[warp][digit_of(k[r], shift)] + rank[r];
                     kout[pos] = k[r];
-                    if (kVals) vout[pos] = vin[i];
                 }
             }
             __syncthreads();   // wcnt is reused by the next chunk
         }
         uint64_t* tk = kin; kin = kout; kout = tk;
-        uint32_t* tv = vin; vin = vout; vout = tv;
         __syncthreads();       // this pass's writes are read by the next pass
     }
     if (kin != keys) {         // odd number of passes: the result is in the temporaries
         for (unsigned i = t; i < n; i += kScThreads) {
             keys[i] = kin[i];
-            if (kVals) vals[i] = vin[i];
         }
     }
 }
@@ -606,41 +587,47 @@ void os_scatter_pass(int byte, unsigned nb, size_t dyn, cudaStream_t st, const u
 
 }  // namespace
 
+// Workspace of the multi-launch passes (no status word): a digit table, its scan, and the scan's own.
 size_t radix_workspace_elems(size_t n) {
-    const size_t nb = (n + kRsTile - 1) / kRsTile;
-    const size_t h = 256 * nb;
-    // the multi-pass layout (two digit tables and a scan) or the single-sweep one (a 64-bit status
-    // word per tile and digit, the histograms and starts of all passes, the tile counter), whichever
-    // is larger, plus alignment slack
-    return std::max(2 * h + scan_workspace_elems(h), 2 * h + 2 * kOsMaxPasses * 256 + 64) + 16;
+    const size_t h = 256 * ((n + kRsTile - 1) / kRsTile);
+    return 2 * h + scan_workspace_elems(h) + 16;
 }
 
-// Sorts (keys, vals) ascending by the low `bits` bits of keys, ping-ponging through
-// keys_tmp/vals_tmp.  vals may be null.  ws: radix_workspace_elems(n) u32.  With a status word
-// (device), arrays of more than kOneSweepMin keys take the single-sweep passes, whose bounded
-// look-back sets kStatusWaitTimeout there if it ever gives up.  With `in_tmp`, a result that ends in
-// the temporaries after an odd number of passes stays there and *in_tmp is set (the caller swaps its
-// buffers); without it the result is copied back into keys/vals.
-constexpr size_t kOneSweepMin = (size_t)1 << 20;
+// Single-sweep passes: the histograms, starts and tile counters of all passes and a 64-bit status word per
+// tile and digit, for all passes of arrays up to kSweepAllPasses (one clearing serves them), else of one.
+constexpr size_t kSweepAllPasses = (size_t)1 << 21;
+static size_t sweep_status_sets(size_t n, int passes) { return n <= kSweepAllPasses ? (size_t)passes : 1; }
+size_t sweep_workspace_elems(size_t n) {
+    const size_t h = 256 * ((n + kRsTile - 1) / kRsTile);
+    return std::max(2 * h * sweep_status_sets(n, kOsMaxPasses) + 2 * kOsMaxPasses * 256 + kOsMaxPasses + 64,
+                    radix_workspace_elems(std::min<size_t>(n, kSmallSort)));
+}
 
+// Sorts (keys, vals) ascending by the low `bits` bits of keys, ping-ponging through keys_tmp/vals_tmp.
+// vals may be null.  With a status word (device) the passes are single-sweep (arrays of keys alone up to
+// kSmallSort: one block), whose bounded look-back sets kStatusWaitTimeout there if it ever gives up, and
+// ws has sweep_workspace_elems(n) u32; without one (keys alone) ws has radix_workspace_elems(n).  With
+// `in_tmp`, a result that ends in the temporaries after an odd number of passes stays there and *in_tmp
+// is set (the caller swaps its buffers); without it the result is copied back into keys/vals.
 void radix_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp, size_t n, int bits,
                 uint32_t* ws, cudaStream_t st, unsigned long long* status, bool* in_tmp) {
     if (in_tmp) *in_tmp = false;
     if (n <= 1 || bits <= 0) return;
     if (n >= (1ull << 32)) fail(-1, "radix_sort: more than 2^32 - 1 keys");
-    if (status && n > kOneSweepMin) {
-        const int passes = (bits + 7) / 8;
+    if (vals && !status) fail(-1, "radix_sort: values need a status word");
+    const int passes = (bits + 7) / 8;
+    if (status && (vals || n > kSmallSort)) {
         // keys alone: 8192-key tiles; with values: 4096-key tiles
         constexpr int kRoundsK = 16, kRoundsV = 8;
         const size_t tile = (size_t)kScThreads * (vals ? kRoundsV : kRoundsK);
         const size_t dyn_k = tile * 8, dyn_kv = tile * 12;
         const unsigned nb = (unsigned)((n + tile - 1) / tile);
-        uint64_t* tstat = (uint64_t*)(((uintptr_t)ws + 15) & ~(uintptr_t)15);   // [nb][256]
-        uint32_t* ghist = (uint32_t*)(tstat + (size_t)nb * 256);                // [passes][256]
-        uint32_t* gstart = ghist + kOsMaxPasses * 256;                           // [passes][256]
-        uint32_t* ctr = gstart + kOsMaxPasses * 256;                              // [passes]
-        TJ_CUDA(cudaMemsetAsync(ghist, 0, (size_t)passes * 256 * sizeof(uint32_t), st));
-        TJ_CUDA(cudaMemsetAsync(ctr, 0, (size_t)passes * sizeof(uint32_t), st));
+        const size_t sets = sweep_status_sets(n, passes), set = (size_t)nb * 256;
+        uint64_t* tstat = (uint64_t*)(((uintptr_t)ws + 15) & ~(uintptr_t)15);   // [sets][nb][256]
+        uint32_t* ghist = (uint32_t*)(tstat + sets * set);                      // [passes][256]
+        uint32_t* ctr = ghist + passes * 256;                                    // [passes]
+        uint32_t* gstart = ctr + passes;                                         // [passes][256]
+        TJ_CUDA(cudaMemsetAsync(tstat, 0, (uint8_t*)gstart - (uint8_t*)tstat, st));
         const unsigned hb = (unsigned)std::min<size_t>((size_t)num_sms() * 4,
                                                        (n + kOsHistThreads * kOsHistKeys - 1) /
                                                            (kOsHistThreads * kOsHistKeys));
@@ -655,13 +642,14 @@ void radix_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* va
         uint64_t *kin = keys, *kout = keys_tmp;
         uint32_t *vin = vals, *vout = vals_tmp;
         for (int p = 0; p < passes; ++p) {
-            TJ_CUDA(cudaMemsetAsync(tstat, 0, (size_t)nb * 256 * sizeof(uint64_t), st));
+            uint64_t* ts = tstat + (sets > 1 ? p * set : 0);
+            if (sets == 1 && p > 0) TJ_CUDA(cudaMemsetAsync(ts, 0, set * sizeof(uint64_t), st));
             if (vals)
-                os_scatter_pass<true, kRoundsV>(p, nb, dyn_kv, st, kin, vin, kout, vout, n, gstart + p * 256, tstat,
+                os_scatter_pass<true, kRoundsV>(p, nb, dyn_kv, st, kin, vin, kout, vout, n, gstart + p * 256, ts,
                                                 ctr + p, status);
             else
                 os_scatter_pass<false, kRoundsK>(p, nb, dyn_k, st, kin, nullptr, kout, nullptr, n, gstart + p * 256,
-                                                 tstat, ctr + p, status);
+                                                 ts, ctr + p, status);
             std::swap(kin, kout);
             std::swap(vin, vout);
         }
@@ -676,48 +664,82 @@ void radix_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* va
         return;
     }
     if (n <= kSmallSort) {
-        const int passes = (bits + 7) / 8;
-        if (vals)
-            launch(rs_small<true>, 1, kScThreads, 0, st, keys, vals, keys_tmp, vals_tmp, (unsigned)n, passes);
-        else
-            launch(rs_small<false>, 1, kScThreads, 0, st, keys, (uint32_t*)nullptr, keys_tmp, (uint32_t*)nullptr,
-                   (unsigned)n, passes);
+        launch(rs_small, 1, kScThreads, 0, st, keys, keys_tmp, (unsigned)n, passes);
         return;
     }
-    const size_t dyn_k = (size_t)kRsTile * 8, dyn_kv = (size_t)kRsTile * 12;
-    TJ_CUDA(cudaFuncSetAttribute(rs_scatter<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_k));
-    TJ_CUDA(cudaFuncSetAttribute(rs_scatter<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    if (vals) {
-        TJ_CUDA(cudaFuncSetAttribute(rs_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_kv));
-        TJ_CUDA(cudaFuncSetAttribute(rs_scatter<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    }
+    const size_t dyn_k = (size_t)kRsTile * 8;
+    TJ_CUDA(cudaFuncSetAttribute(rs_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_k));
+    TJ_CUDA(cudaFuncSetAttribute(rs_scatter, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     const unsigned nb = (unsigned)((n + kRsTile - 1) / kRsTile);
     const size_t h = 256 * (size_t)nb;
     uint32_t* hist = ws;
     uint32_t* offs = ws + h;
     uint32_t* sws = ws + 2 * h;
-    const int passes = (bits + 7) / 8;
     uint64_t *kin = keys, *kout = keys_tmp;
-    uint32_t *vin = vals, *vout = vals_tmp;
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
         launch(rs_hist, nb, kRsThreads, 0, st, kin, n, shift, hist, nb);
         exclusive_scan_u32(hist, offs, h, nullptr, sws, st);
-        if (vals)
-            launch(rs_scatter<true>, nb, kScThreads, dyn_kv, st, kin, vin, kout, vout, n, shift, offs, nb);
-        else
-            launch(rs_scatter<false>, nb, kScThreads, dyn_k, st, kin, nullptr, kout, nullptr, n, shift, offs, nb);
+        launch(rs_scatter, nb, kScThreads, dyn_k, st, kin, kout, n, shift, offs, nb);
         std::swap(kin, kout);
-        std::swap(vin, vout);
     }
-    if (kin != keys) {
-        cudaMemcpyAsync(keys, kin, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st);
-        if (vals) cudaMemcpyAsync(vals, vin, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+    if (kin != keys) cudaMemcpyAsync(keys, kin, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st);
+}
+
+// ------------------------------------------------------------------ segment sort
+namespace {
+
+// One block per segment: keys (the low 32 bits differ inside a segment) with the row's number in it below,
+// by a bitonic network in shared memory; equal keys keep their order.  One launch orders the rows of any
+// number of small joins, where the radix passes take a dozen per side.
+constexpr int kSegThreads = 1024;
+__global__ void __launch_bounds__(kSegThreads) seg_sort(uint64_t* keys, uint32_t* perm, uint32_t* local,
+                                                        const long long* off, long long n) {
+    extern __shared__ uint64_t seg[];
+    const long long b = off ? off[blockIdx.x] : 0, e = off ? off[blockIdx.x + 1] : n;
+    const unsigned len = (unsigned)(e - b);
+    if (len == 0) return;
+    const uint64_t high = keys[b] & 0xFFFFFFFF00000000ull;
+    unsigned m = 2;
+    while (m < len) m <<= 1;
+    for (unsigned i = threadIdx.x; i < m; i += kSegThreads)
+        seg[i] = i < len ? (keys[b + i] << 32) | i : ~0ull;
+    __syncthreads();
+    for (unsigned k = 2; k <= m; k <<= 1)
+        for (unsigned s = k >> 1; s > 0; s >>= 1) {
+            for (unsigned i = threadIdx.x; i < m / 2; i += kSegThreads) {
+                const unsigned x = 2 * i - (i & (s - 1)), y = x + s;   // the pair of step s
+                const uint64_t u = seg[x], v = seg[y];
+                if ((u > v) == ((x & k) == 0)) {
+                    seg[x] = v;
+                    seg[y] = u;
+                }
+            }
+            // steps of less than 32 stay within a warp's own 64 elements
+            if (s > 32 || k == m || s == 1) __syncthreads();
+            else __syncwarp();
+        }
+    for (unsigned i = threadIdx.x; i < len; i += kSegThreads) {
+        const uint64_t w = seg[i];
+        keys[b + i] = high | (w >> 32);
+        perm[b + i] = (uint32_t)b + (uint32_t)w;
+        if (local) local[b + i] = (uint32_t)w;
     }
+}
+
+}  // namespace
+
+void segment_sort(uint64_t* keys, uint32_t* perm, uint32_t* local, const long long* off, int nseg, long long n,
+                  long long longest, cudaStream_t st) {
+    size_t m = 2;
+    while ((long long)m < longest) m <<= 1;
+    if (longest > kSegmentSort) fail(-1, "segment_sort: segment too long");
+    TJ_CUDA(cudaFuncSetAttribute(seg_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(m * 8)));
+    launch(seg_sort, (unsigned)nseg, kSegThreads, m * 8, st, keys, perm, local, off, n);
 }
 
 int radix_passes(int bits) { return (bits + 7) / 8; }
 
-bool radix_result_in_tmp(size_t n, int bits) { return n > kOneSweepMin && radix_passes(bits) % 2 == 1; }
+bool radix_result_in_tmp(size_t n, int bits) { return n > kSmallSort && radix_passes(bits) % 2 == 1; }
 
 }  // namespace tj
