@@ -740,8 +740,9 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         std::vector<HalfView> hv(ncls);
         for (int c = 0; c < ncls; ++c) {
             Cls& K = *C[c];
-            TileSet& H = K.tSh;
-            if (!H.built) {   // halves not made by the fused operand pass
+            // a self-join's halves are its R tiles
+            TileSet& H = self && !K.tSh.built ? K.tR : K.tSh;
+            if (&H == &K.tSh && !H.built) {   // halves not made by the fused operand pass
                 for (size_t t = 0; t < K.tS.h_row0.size(); ++t)
                     for (uint32_t h = 0; h < 2; ++h) {
                         const uint32_t nv = K.tS.h_nvalid[t];
@@ -754,7 +755,12 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
             hv[c] = HalfView{K.tR.ctrT.p, K.tR.loT.p, K.tR.hiT.p, K.tR.rad.p, H.ctrR.p, H.loR.p, H.hiR.p, H.rad.p,
                              H.nvalid.p, K.tR.ntiles, H.ntiles, g.rbase[c], g.sbase[c], cls_d[c], 0};
         }
-        half_masks(hv, cand, g.ntR_total, d_rt.p, d_jps.p, self, st);
+        unsigned long long full = 0;
+        if (nj == 1) {
+            for (long long I = 0; I < g.ntR_total; ++I)   // S tiles above the diagonal of R tile I, or all
+                full += (unsigned long long)(g.ntS_total - (self ? std::min<long long>(g.ntS_total, (I * kTileR + 1) / kTileS) : 0));
+        }
+        half_masks(hv, cand, g.ntR_total, d_rt.p, d_jps.p, self, full, st);
     }
     launch(pairs_screened_kernel, num_sms() * 4, 256, 0, st, (const uint4*)cand.chunks.p,
            (const uint32_t*)(cand.dev_counts.p + 1), (const uint32_t*)cand.jlist.p, (const uint4*)d_rt.p,

@@ -1496,7 +1496,61 @@ __global__ void __launch_bounds__(256) zero_tail(uint16_t* op, int opw, double* 
     }
 }
 
-// Candidate test: thread = one S tile J, 16 R tiles per block (from shared memory).
+// Candidate test: thread = one S tile J, kCandI R tiles per block.  The block's R tiles lie in shared
+// memory as [k][statistic][tile], so that four tiles' values come in one 16-byte broadcast (read one by one
+// they were half of the instructions and paced the test): sums of both bounds, in FP32.
+template <int kCandI>
+TJ_DEV void tile_bounds(const float* sm, const float* ctrT, const float* loT, const float* hiT, size_t pitch, size_t j,
+                        int d, float (&ball)[kCandI], float (&box)[kCandI]) {
+#pragma unroll
+    for (int ii = 0; ii < kCandI; ++ii) ball[ii] = box[ii] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < d; ++k) {
+        const float cj = ctrT[(size_t)k * pitch + j];
+        const float lj = loT[(size_t)k * pitch + j];
+        const float hj = hiT[(size_t)k * pitch + j];
+        const float* row = sm + (size_t)k * 3 * kCandI;
+        constexpr int kV = kCandI < 4 ? kCandI : 4;
+#pragma unroll
+        for (int i0 = 0; i0 < kCandI; i0 += kV) {
+            float c[kV], lo[kV], hi[kV];
+            if (kV == 4) {
+                *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(row + i0);
+                *reinterpret_cast<float4*>(lo) = *reinterpret_cast<const float4*>(row + kCandI + i0);
+                *reinterpret_cast<float4*>(hi) = *reinterpret_cast<const float4*>(row + 2 * kCandI + i0);
+            } else {
+#pragma unroll
+                for (int v = 0; v < kV; ++v) {
+                    c[v] = row[i0 + v];
+                    lo[v] = row[kCandI + i0 + v];
+                    hi[v] = row[2 * kCandI + i0 + v];
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < kV; ++v) {
+                const float dc = c[v] - cj;
+                ball[i0 + v] = fmaf(dc, dc, ball[i0 + v]);
+                const float gap = fmax3(lj - hi[v], lo[v] - hj, 0.f);
+                box[i0 + v] = fmaf(gap, gap, box[i0 + v]);
+            }
+        }
+    }
+}
+template <int kCandI>
+TJ_DEV void stage_rtiles(float* sm, const float* ctrT, const float* loT, const float* hiT, int ntR, int I0, int nI,
+                         int d) {
+    for (int e = threadIdx.x; e < kCandI * d; e += blockDim.x) {
+        const int k = e / kCandI, ii = e % kCandI;
+        const bool ok = ii < nI;
+        const size_t at = (size_t)k * ntR + I0 + ii;
+        float* row = sm + (size_t)k * 3 * kCandI + ii;
+        row[0] = ok ? ctrT[at] : 0.f;
+        row[kCandI] = ok ? loT[at] : 0.f;
+        row[2 * kCandI] = ok ? hiT[at] : 0.f;
+    }
+    __syncthreads();
+}
+
 // Keeps (I, J) unless a rigorous lower bound on every pair distance exceeds sqrt(Tp).
 template <int kCandI>
 __global__ void __launch_bounds__(256) cand_test(const float* rctrT, const float* rloT, const float* rhiT,
@@ -1504,50 +1558,31 @@ __global__ void __launch_bounds__(256) cand_test(const float* rctrT, const float
                                                  const float* sloT, const float* shiT, const float* srad, int ntS,
                                                  int d, int tileR, int tileS, double Tp, int self_join,
                                                  uint32_t* bitmap, int words) {
-    extern __shared__ float sm[];   // [3][kCandI][d]
-    float* sc = sm;
-    float* slo = sm + kCandI * d;
-    float* shi = sm + 2 * kCandI * d;
+    extern __shared__ __align__(16) float sm[];   // [d][3][kCandI]
     const int I0 = blockIdx.y * kCandI;
     const int nI = min(kCandI, ntR - I0);
-    for (int e = threadIdx.x; e < kCandI * d; e += blockDim.x) {
-        const int ii = e / d, k = e % d;
-        const bool ok = ii < nI;
-        sc[e] = ok ? rctrT[(size_t)k * ntR + I0 + ii] : 0.f;
-        slo[e] = ok ? rloT[(size_t)k * ntR + I0 + ii] : 0.f;
-        shi[e] = ok ? rhiT[(size_t)k * ntR + I0 + ii] : 0.f;
-    }
-    __syncthreads();
     const int J = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lane = threadIdx.x & 31;
+    // self-joins: some column of J must exceed some row of I (sorted positions); a block with no such pair
+    // only clears its words
+    if (self_join && (long long)min((int)(blockIdx.x + 1) * (int)blockDim.x, ntS) * tileS - 1 <= (long long)I0 * tileR) {
+        if (lane == 0 && (J >> 5) < words)
+            for (int ii = 0; ii < nI; ++ii) bitmap[(size_t)(I0 + ii) * words + (J >> 5)] = 0;
+        return;
+    }
+    stage_rtiles<kCandI>(sm, rctrT, rloT, rhiT, ntR, I0, nI, d);
     const bool jok = J < ntS;
     float ball[kCandI], box[kCandI];
-#pragma unroll
-    for (int ii = 0; ii < kCandI; ++ii) ball[ii] = box[ii] = 0.f;
-    if (jok) {
-        for (int k = 0; k < d; ++k) {
-            const float cj = sctrT[(size_t)k * ntS + J];
-            const float lj = sloT[(size_t)k * ntS + J];
-            const float hj = shiT[(size_t)k * ntS + J];
-#pragma unroll
-            for (int ii = 0; ii < kCandI; ++ii) {
-                const float dc = sc[ii * d + k] - cj;
-                ball[ii] = fmaf(dc, dc, ball[ii]);
-                const float gap = fmaxf(fmaxf(lj - shi[ii * d + k], slo[ii * d + k] - hj), 0.f);
-                box[ii] = fmaf(gap, gap, box[ii]);
-            }
-        }
-    }
+    tile_bounds<kCandI>(sm, sctrT, sloT, shiT, ntS, jok ? J : ntS - 1, d, ball, box);
     // FP32 sums of d non-negative terms: computed >= (1 - (d+4) 2^-23) * true  => true >= computed * f
     const float f = 1.f - (float)(d + 8) * 0x1p-23f;
     const float rtp = (float)(sqrt(Tp) * (1.0 + 0x1p-20));
     const float tpf = (float)(Tp * (1.0 + 0x1p-20));
     const float rj = jok ? srad[J] : 0.f;
-    const unsigned lane = threadIdx.x & 31;
     for (int ii = 0; ii < kCandI; ++ii) {
         const int I = I0 + ii;
         bool keep = jok && ii < nI;
         if (keep && self_join) {
-            // some column index of J must exceed some row index of I (sorted positions)
             const long long maxcol = (long long)(J + 1) * tileS - 1;
             keep = maxcol > (long long)I * tileR;
         }
@@ -1566,22 +1601,12 @@ __global__ void __launch_bounds__(256) cand_test(const float* rctrT, const float
 template <int kCandI>
 __global__ void __launch_bounds__(256) cand_test_batched(const CandBlock* blocks, const CandClassView* views,
                                                          const double* Tp_blk, uint32_t* bitmap, int words) {
-    extern __shared__ float sm[];   // [3][kCandI][d]
+    extern __shared__ __align__(16) float sm[];   // [d][3][kCandI]
     const CandBlock cb = blocks[blockIdx.x];
     const CandClassView cv = views[cb.cls];
     const int d = cv.d;
-    float* sc = sm;
-    float* slo = sm + kCandI * d;
-    float* shi = sm + 2 * kCandI * d;
     const int iloc0 = (int)cb.i0 - cv.rbase;   // class-local R tile of the block's first tile
-    for (int e = threadIdx.x; e < kCandI * d; e += blockDim.x) {
-        const int ii = e / d, k = e % d;
-        const bool ok = ii < (int)cb.ni;
-        sc[e] = ok ? cv.rctrT[(size_t)k * cv.ntR + iloc0 + ii] : 0.f;
-        slo[e] = ok ? cv.rloT[(size_t)k * cv.ntR + iloc0 + ii] : 0.f;
-        shi[e] = ok ? cv.rhiT[(size_t)k * cv.ntR + iloc0 + ii] : 0.f;
-    }
-    __syncthreads();
+    stage_rtiles<kCandI>(sm, cv.rctrT, cv.rloT, cv.rhiT, cv.ntR, iloc0, (int)cb.ni, d);
     const double Tp = Tp_blk[blockIdx.x];
     const float f = 1.f - (float)(d + 8) * 0x1p-23f;
     const float rtp = (float)(sqrt(Tp) * (1.0 + 0x1p-20));
@@ -1589,26 +1614,12 @@ __global__ void __launch_bounds__(256) cand_test_batched(const CandBlock* blocks
     const unsigned lane = threadIdx.x & 31;
     for (int j0 = 0; j0 < (int)cb.nj; j0 += blockDim.x) {
         const int jl = j0 + threadIdx.x;          // S tile index inside the join
+        if (j0 + (int)(threadIdx.x & ~31u) >= (int)cb.nj) continue;   // warp-uniform: no tile for this warp
         const bool jok = jl < (int)cb.nj;
-        const int js = (int)cb.j0 - cv.sbase + jl;   // class-local S tile
+        const int js = (int)cb.j0 - cv.sbase + min(jl, (int)cb.nj - 1);   // class-local S tile
         float ball[kCandI], box[kCandI];
-#pragma unroll
-        for (int ii = 0; ii < kCandI; ++ii) ball[ii] = box[ii] = 0.f;
-        if (jok) {
-            for (int k = 0; k < d; ++k) {
-                const float cj = cv.sctrT[(size_t)k * cv.ntS + js];
-                const float lj = cv.sloT[(size_t)k * cv.ntS + js];
-                const float hj = cv.shiT[(size_t)k * cv.ntS + js];
-#pragma unroll
-                for (int ii = 0; ii < kCandI; ++ii) {
-                    const float dc = sc[ii * d + k] - cj;
-                    ball[ii] = fmaf(dc, dc, ball[ii]);
-                    const float gap = fmaxf(fmaxf(lj - shi[ii * d + k], slo[ii * d + k] - hj), 0.f);
-                    box[ii] = fmaf(gap, gap, box[ii]);
-                }
-            }
-        }
-        const float rj = jok ? cv.srad[js] : 0.f;
+        tile_bounds<kCandI>(sm, cv.sctrT, cv.sloT, cv.shiT, cv.ntS, js, d, ball, box);
+        const float rj = cv.srad[js];
         for (int ii = 0; ii < kCandI; ++ii) {
             bool keep = jok && ii < (int)cb.ni;
             if (keep) {
@@ -1722,17 +1733,21 @@ __global__ void __launch_bounds__(1024) place_chunks(const uint32_t* cnt, const 
 // tile I with cand_test's rigorous ball and box bounds (on the halves' own statistics) and stores the
 // live halves in bits 30-31 of the jlist entry.  The screen then issues and tests only live halves,
 // packing them densely into its MMA and epilogue pipeline; an entry whose halves are both dead is
-// skipped.  Warps stride over the scheduling chunks (at most chunk_items candidates of one R tile),
+// skipped.  Where no tile pair of the join was ruled out by the candidate test (`full` candidates), halves
+// are not either, but for a few that are not worth 470 us (60,000 x 512): only those with no row, or below a
+// self-join's diagonal, are dropped.  Warps stride over the scheduling chunks (at most chunk_items candidates of one R tile),
 // the chunk's R tile statistics in the warp's shared memory, and take its candidates one at a time
 // with the lanes over the dimensions; the halves' statistics are read row-major, so each load of
 // the warp is one contiguous run of a candidate's row.
 __global__ void __launch_bounds__(256) half_mask_kernel(const uint4* chunks, const uint32_t* nchunks, uint32_t* jlist,
                                                         const uint4* rtiles, const JoinParams* jps,
-                                                        const HalfView* views, int self_join, int dmax) {
+                                                        const HalfView* views, int self_join, int dmax,
+                                                        const uint32_t* total, uint32_t full) {
     extern __shared__ float hm_sm[];   // [8 warps][3][dmax]: R tile centroid, low, high
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* rs = hm_sm + (size_t)warp * 3 * dmax;
     const unsigned nch = *nchunks;
+    const bool dense = full != 0 && *total == full;
     for (unsigned ci = blockIdx.x * 8 + warp; ci < nch; ci += gridDim.x * 8) {   // warp-uniform
         const uint4 ch = chunks[ci];
         const int I = (int)ch.x;
@@ -1740,6 +1755,19 @@ __global__ void __launch_bounds__(256) half_mask_kernel(const uint4* chunks, con
         const HalfView v = views[rt.w];
         const int d = v.d;
         const int il = I - v.rbase;   // class-local R tile
+        if (dense) {
+            for (uint32_t e = ch.y + lane; e < ch.z; e += 32) {
+                const uint32_t J = jlist[e] & kJMask;
+                const int h0 = 2 * ((int)J - v.sbase);
+                unsigned mask = 0;
+                for (int h = 0; h < 2; ++h)
+                    if (h0 + h < v.ntH && v.hnv[h0 + h] != 0 &&
+                        !(self_join && (long long)(h0 + h) * 128 + 127 <= (long long)il * 128))
+                        mask |= 1u << h;
+                jlist[e] = J | (mask << 30);
+            }
+            continue;
+        }
         __syncwarp();                  // the previous chunk's reads of rs are done
         for (int k = lane; k < d; k += 32) {
             rs[k] = v.rctrT[(size_t)k * v.ntR + il];
@@ -2161,7 +2189,7 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
 }
 
 void half_masks(const std::vector<HalfView>& views, const Candidates& c, int ntR_total, const uint4* rtiles,
-                const JoinParams* jps, bool self_join, cudaStream_t st) {
+                const JoinParams* jps, bool self_join, unsigned long long full, cudaStream_t st) {
     if (ntR_total == 0 || views.empty()) return;
     int dmax = 1;
     for (const auto& v : views) dmax = std::max(dmax, v.d);
@@ -2174,7 +2202,7 @@ void half_masks(const std::vector<HalfView>& views, const Candidates& c, int ntR
     const unsigned blocks = (unsigned)std::min<size_t>((size_t)num_sms() * 8, (c.chunks_cap + 7) / 8);
     launch(half_mask_kernel, std::max(1u, blocks), 256, smem, st, (const uint4*)c.chunks.p,
            (const uint32_t*)(c.dev_counts.p + 1), c.jlist.p, rtiles, jps, (const HalfView*)dv.p, self_join ? 1 : 0,
-           dmax);
+           dmax, (const uint32_t*)c.dev_counts.p, (uint32_t)(full < 0xFFFFFFFFull ? full : 0));
 }
 
 void tile_stats_rowmajor(TileSet& ts, cudaStream_t st) {

@@ -263,9 +263,10 @@ struct HalfView {
     const uint32_t* hnv;   // [ntH] rows of each half that are real points
     int ntR, ntH, rbase, sbase, d, pad;
 };
-// Marks the live 128-row halves of every candidate's S tile in bits 30-31 of its jlist entry.
+// Marks the live 128-row halves of every candidate's S tile in bits 30-31 of its jlist entry.  `full`:
+// candidates if no tile pair is ruled out (0: not known).
 void half_masks(const std::vector<HalfView>& views, const Candidates& c, int ntR_total, const uint4* rtiles,
-                const JoinParams* jps, bool self_join, cudaStream_t st);
+                const JoinParams* jps, bool self_join, unsigned long long full, cudaStream_t st);
 // Row-major copies (ctrR, loR, hiR) of a tile set's centroids and boxes.
 void tile_stats_rowmajor(TileSet& ts, cudaStream_t st);
 constexpr uint32_t kJMask = 0x3FFFFFFFu;   // jlist entry: S tile id in the low 30 bits
