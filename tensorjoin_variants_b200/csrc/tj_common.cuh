@@ -288,9 +288,19 @@ TJ_DEV bool mbar_try_wait_cluster(uint64_t* bar, unsigned parity) {
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+TJ_DEV bool mbar_test_cluster(uint64_t* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // bounded wait with cluster-scope acquire (a barrier that the other CTA of the pair arrives on)
 TJ_DEV bool mbar_wait_cluster(uint64_t* bar, unsigned parity, unsigned long long* status,
                               unsigned long long limit_ns = kWaitLimitNs) {
+    if (mbar_test_cluster(bar, parity)) return true;
     const int spins = limit_ns >= 1000000ull ? 256 : 1;
     for (int it = 0; it < spins; ++it)
         if (mbar_try_wait_cluster(bar, parity)) return true;

@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
     } else if (warp == 1) {
         // ------------------------------------------------------------ UMMA issuer (pair: CTA 0 only)
         if (lane == 0 && rank == 0) {
+            const uint32_t smem_lo = ((smem_u32(smem) >> 4) & 0x3FFFu) | (1u << 16);
             unsigned stage = 0, phase = 0, acc = 0, acc_phase = 0;
             unsigned long long n_mma = 0;   // items issued
             unsigned ns = 0;                // one SM: half-items issued
@@ -461,6 +462,7 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                 const ScreenClassArgs& ca = a.cls[rt.w];
                 const int kblocks = ca.kblocks, ksteps = ca.kbk / 16;
                 const uint32_t dh = ca.desc_hi;
+                auto desc = [dh](uint32_t lo) { return ((uint64_t)dh << 32) | lo; };
                 for (unsigned e = e0; e < e1 && ok; ++e) {
                     unsigned hm = 3u;   // one SM: live 128-row halves of the item's S tile
                     if (!kPair && a.half) {
@@ -488,32 +490,35 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                     tc_fence_after();
                     const unsigned d_tmem = tmem + acc * kTileS;                 // pair: 256 columns
                     const unsigned d0 = tmem + bh[0] * 128u, d1 = tmem + bh[1] * 128u;   // one SM: 2 x 128
-                    const unsigned bhalf = 256u * (unsigned)ca.kbk;              // bytes of 128 B rows
+                    const unsigned bhalf = 16u * (unsigned)ca.kbk;               // 128 B rows, in 16 bytes
                     for (int kb = 0; kb < kblocks; ++kb) {
                         const long long t_o = kTimes ? clock64() : 0;
                         if (!mbar_wait(&ctl->full[stage], phase, status, a.wait_ns)) { ok = false; break; }
                         if (kTimes) w_op += clock64() - t_o;
                         if (*(volatile int*)&ctl->abort_flag) { ok = false; break; }
                         tc_fence_after();
-                        const uint8_t* sa = smem + (size_t)stage * kStageBytes;
+                        // descriptors: a constant or a half's offset added to the low word of the stage's (built
+                        // from pointers, with their conversions, they were most of what the issuing thread did, and
+                        // it paced the screen: 70 to 90 % of its time went by outside its waits)
+                        const uint32_t sl = smem_lo + stage * (kStageBytes >> 4);
 #pragma unroll
                         for (int k = 0; k < kBK / 16; ++k) {
                             if (k >= ksteps) break;
                             const unsigned accum = (kb | k) != 0 ? 1u : 0u;
-                            const uint64_t ad = desc_kmajor(sa, k * 32, dh);
+                            const uint64_t ad = desc(sl + 2 * k);
                             if (kPair) {
-                                umma_f16_pair(d_tmem, ad, desc_kmajor(sa + Cfg::kBhi, k * 32, dh), a.idesc_pair, accum);
+                                umma_f16_pair(d_tmem, ad, desc(sl + (Cfg::kBhi >> 4) + 2 * k), a.idesc_pair, accum);
                             } else {
 #pragma unroll
                                 for (int h = 0; h < 2; ++h) {
                                     if (!((hm >> h) & 1u)) continue;
                                     const unsigned dd = h ? d1 : d0;
-                                    const uint64_t bd = desc_kmajor(sa + Cfg::kBhi + h * bhalf, k * 32, dh);
+                                    const uint32_t bo = (h ? bhalf : 0u) + 2 * k;
+                                    const uint64_t bd = desc(sl + (Cfg::kBhi >> 4) + bo);
                                     umma_f16(dd, ad, bd, a.idesc, accum);
                                     if (kSplit) {   // z.w ~ hi.hi + hi.lo + lo.hi, one FP32 accumulator
-                                        umma_f16(dd, ad, desc_kmajor(sa + Cfg::kBlo + h * bhalf, k * 32, dh), a.idesc,
-                                                 1u);
-                                        umma_f16(dd, desc_kmajor(sa + Cfg::kAlo, k * 32, dh), bd, a.idesc, 1u);
+                                        umma_f16(dd, ad, desc(sl + (Cfg::kBlo >> 4) + bo), a.idesc, 1u);
+                                        umma_f16(dd, desc(sl + (Cfg::kAlo >> 4) + 2 * k), bd, a.idesc, 1u);
                                     }
                                 }
                             }
