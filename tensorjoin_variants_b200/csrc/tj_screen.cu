@@ -94,10 +94,12 @@ struct ColMetaF : ColMetaHot {
 };
 static_assert(sizeof(ColMetaF) % 16 == 0 && sizeof(ColMetaHot) % 16 == 0, "16-byte aligned parts");
 
-template <int kStages>
+constexpr int kMaxRing = 8;   // operand stages at most
 struct ScreenCtl {
-    uint64_t full[kStages];
-    uint64_t empty[kStages];
+    uint64_t full[kMaxRing];
+    uint64_t empty[kMaxRing];
+    uint64_t a_full[2];         // CTA pair: resident R tiles
+    uint64_t a_empty[2];
     uint64_t acc_full[kAccMax];
     uint64_t acc_empty[kAccMax];
     uint64_t meta_full[kMetaSlots];
@@ -135,7 +137,7 @@ template <int kSplit, bool kPair>
 constexpr size_t screen_smem() {
     using Cfg = typename StageSel<kSplit, kPair>::type;
     return 1024 + (size_t)Cfg::kStages * Cfg::kBytes + (size_t)kMetaSlots * sizeof(ColMetaHot) +
-           sizeof(ScreenCtl<Cfg::kStages>);
+           sizeof(ScreenCtl);
 }
 static_assert(screen_smem<0, false>() <= 232448 && screen_smem<1, false>() <= 232448 &&
               screen_smem<0, true>() <= 232448, "227 KB of shared memory per CTA at most");
@@ -170,7 +172,7 @@ struct ScreenArgs {
     const JoinParams* jps;     // per join
     ScreenClassArgs cls[kMaxClass];
     int ncls;
-    unsigned idesc;
+    unsigned idesc, idesc2;
     // CTA-pair mode: every (R tile, S tile) pair is a candidate; chunks are generated from the grid
     unsigned idesc_pair;       // M = 256 instruction descriptor
     unsigned ntR, ntS, nT;     // R tiles, S tiles, R tile pairs
@@ -192,14 +194,15 @@ struct ScreenArgs {
     unsigned long long* role_t;   // [kRoleSlots] SM clock cycles per role and wait, summed over CTAs
     unsigned njoins;
     int nstages;                  // operand stages in the ring (<= the compiled count; a tuning knob)
+    int na;                       // CTA pair: buffers of a chunk's resident R tile (0: R streams with S)
+    unsigned abytes, stage_bytes; // bytes of such a buffer, and of a stage beside it
     int half;                     // one SM: jlist entries carry live-half masks in bits 30-31
 };
 
 // One SM: the producer publishes the chunks it takes from the queue in a ring of kChunkRing slots;
 // the UMMA issuer and every epilogue warp read them in the same order (kNoChunk ends the sequence).
 // Its waits are bounded like every other pipeline wait.
-template <int kStages>
-TJ_DEV bool publish_chunk(ScreenCtl<kStages>* ctl, unsigned long long q, unsigned c, unsigned long long* status,
+TJ_DEV bool publish_chunk(ScreenCtl* ctl, unsigned long long q, unsigned c, unsigned long long* status,
                           unsigned long long wait_ns) {
     const unsigned slot = (unsigned)(q % kChunkRing), ph = (unsigned)((q / kChunkRing) & 1);
     if (!mbar_wait(&ctl->cempty[slot], ph ^ 1u, status, wait_ns)) return false;
@@ -208,8 +211,7 @@ TJ_DEV bool publish_chunk(ScreenCtl<kStages>* ctl, unsigned long long q, unsigne
     return true;
 }
 // warp-collective in the epilogue warps (every lane reads; lane 0 frees the slot), one lane elsewhere
-template <int kStages>
-TJ_DEV bool take_chunk(ScreenCtl<kStages>* ctl, unsigned long long q, unsigned& c, unsigned long long* status,
+TJ_DEV bool take_chunk(ScreenCtl* ctl, unsigned long long q, unsigned& c, unsigned long long* status,
                        unsigned long long wait_ns, bool warp_collective) {
     const unsigned slot = (unsigned)(q % kChunkRing), ph = (unsigned)((q / kChunkRing) & 1);
     bool got = mbar_wait(&ctl->cfull[slot], ph, status, wait_ns);
@@ -289,15 +291,19 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     ColMetaHot* meta = (ColMetaHot*)(smem + (size_t)kStages * kStageBytes);
     __shared__ long long role_acc[kScreenThreads / 32][6];   // stall accounting per warp (TJ_FLAG_SCREEN_TIMES)
-    ScreenCtl<kStages>* ctl = (ScreenCtl<kStages>*)(meta + kMetaSlots);
+    ScreenCtl* ctl = (ScreenCtl*)(meta + kMetaSlots);
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned long long* status = &a.ctr->status;
     const unsigned rank = kPair ? cluster_ctarank() : 0u;   // 0: the pair's MMA-issuing CTA
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kMaxRing; ++s) {
             mbar_init(&ctl->full[s], 1);
             mbar_init(&ctl->empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&ctl->a_full[b], 1);
+            mbar_init(&ctl->a_empty[b], 1);
         }
         for (int b = 0; b < kAccMax; ++b) {
             mbar_init(&ctl->acc_full[b], 1);
@@ -332,7 +338,12 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
     tc_fence_after();
     const unsigned tmem = ctl->tmem_base;
     const unsigned nchunks = kPair ? a.nT * ((a.ntS + 63u) / 64u) : *a.nchunks;
-    const int nst = (a.nstages >= 2 && a.nstages <= kStages) ? a.nstages : kStages;
+    // pair, a.na > 0: the R tile of a chunk stays in one of na buffers ahead of the ring, and a stage holds a
+    // k-block of the S side alone; otherwise a stage holds both sides, [A | B]
+    const unsigned na = kPair ? (unsigned)a.na : 0u;
+    const unsigned nst = na || (a.nstages >= 2 && a.nstages <= kStages) ? a.nstages : kStages;
+    uint8_t* ring = smem + (size_t)na * a.abytes;
+    const unsigned stage_bytes = na ? a.stage_bytes : kStageBytes;
     const unsigned cfirst = kPair ? (blockIdx.x >> 1) : blockIdx.x;
     const unsigned cstride = kPair ? (gridDim.x >> 1) : gridDim.x;
     if (a.cta_t && threadIdx.x == 0) a.cta_t[2 * blockIdx.x] = global_ns();
@@ -342,6 +353,7 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
         if (lane == 0) {
             unsigned stage = 0, phase = 0;
             unsigned long long n = 0;   // items issued
+            unsigned n_a = 0;           // R tiles brought in
             bool ok = true;
             const long long t_role = kTimes ? clock64() : 0;
             long long w_stage = 0, w_meta = 0;
@@ -366,6 +378,15 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                 const unsigned tx = a.cls[cls].tx_bytes;
                 const CUtensorMap* mA = &tm.a[cls];
                 const CUtensorMap* mB = &tm.b[cls];
+                if (na) {   // both CTAs' copies complete on the MMA CTA's barrier
+                    const unsigned ab = (unsigned)qc % na;
+                    if (!mbar_wait(&ctl->a_empty[ab], (((unsigned)qc / na) & 1u) ^ 1u, status, a.wait_ns)) { ok = false; break; }
+                    const unsigned fb = mapa_shared(&ctl->a_full[ab], 0);
+                    if (rank == 0) mbar_arrive_expect_tx(&ctl->a_full[ab], 512u * (unsigned)kpad);
+                    for (int kb = 0; kb < kblocks; ++kb)
+                        tma_load_2d_pair(smem + (size_t)ab * a.abytes + kb * (256 * kbk), mA, fb, kb * kbk, rrow);
+                    n_a = (unsigned)qc + 1;
+                }
                 for (unsigned e = e0; e < e1 && ok; ++e) {
                     unsigned J = e, hm = 3u;   // one SM: live 128-row halves of the S tile
                     if (!kPair) {
@@ -387,12 +408,12 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                         if (!mbar_wait(&ctl->empty[stage], phase ^ 1, status, a.wait_ns)) { ok = false; break; }
                         if (kTimes) w_stage += clock64() - t_s;
                         if (*(volatile int*)&ctl->abort_flag) { ok = false; break; }
-                        uint8_t* sa = smem + (size_t)stage * kStageBytes;
+                        uint8_t* sa = ring + (size_t)stage * stage_bytes;
                         if (kPair) {   // both CTAs' copies complete on the MMA CTA's barrier
                             const unsigned fb = mapa_shared(&ctl->full[stage], 0);
-                            if (rank == 0) mbar_arrive_expect_tx(&ctl->full[stage], 2 * tx);
-                            tma_load_2d_pair(sa, mA, fb, kb * kbk, rrow);
-                            tma_load_2d_pair(sa + Cfg::kBhi, mB, fb, kb * kbk, srow);
+                            if (rank == 0) mbar_arrive_expect_tx(&ctl->full[stage], na ? tx : 2 * tx);
+                            if (!na) tma_load_2d_pair(sa, mA, fb, kb * kbk, rrow);
+                            tma_load_2d_pair(na ? sa : sa + Cfg::kBhi, mB, fb, kb * kbk, srow);
                         } else {   // A, then each live 128-row half of B (hi, and lo with the split)
                             const unsigned bhalf = 256u * (unsigned)kbk;
                             mbar_arrive_expect_tx(&ctl->full[stage],
@@ -425,10 +446,16 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
             // released by the pair's MMA (its `empty` barriers, signalled after the MMA that read
             // the copy); where the MMA stopped early these waits run out after kDrainLimitNs each,
             // long after any copy issued has landed.  The final cluster barrier follows both.
-            for (int s = 0; s < nst; ++s) {
-                const unsigned ph = ((unsigned)s < stage) ? phase : (phase ^ 1u);
+            for (unsigned s = 0; s < nst; ++s) {
+                const unsigned ph = (s < stage) ? phase : (phase ^ 1u);
                 if (rank == 0) mbar_wait(&ctl->full[s], ph, status, kDrainLimitNs);
                 else if (n > 0) mbar_wait(&ctl->empty[s], ph, status, kDrainLimitNs);
+            }
+            for (unsigned ab = 0; ab < na; ++ab) {
+                if (n_a <= ab) continue;
+                const unsigned ph = ((n_a - 1 - ab) / na) & 1u;   // the last tile in this buffer
+                if (rank == 0) mbar_wait(&ctl->a_full[ab], ph, status, kDrainLimitNs);
+                else mbar_wait(&ctl->a_empty[ab], ph, status, kDrainLimitNs);
             }
             for (int s = 0; s < kMetaSlots; ++s) {
                 if (n <= (unsigned long long)s) continue;
@@ -440,6 +467,7 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
         // ------------------------------------------------------------ UMMA issuer (pair: CTA 0 only)
         if (lane == 0 && rank == 0) {
             const uint32_t smem_lo = ((smem_u32(smem) >> 4) & 0x3FFFu) | (1u << 16);
+            const uint32_t ring_lo = smem_lo + na * (a.abytes >> 4);
             unsigned stage = 0, phase = 0, acc = 0, acc_phase = 0;
             unsigned long long n_mma = 0;   // items issued
             unsigned ns = 0;                // one SM: half-items issued
@@ -463,6 +491,9 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                 const int kblocks = ca.kblocks, ksteps = ca.kbk / 16;
                 const uint32_t dh = ca.desc_hi;
                 auto desc = [dh](uint32_t lo) { return ((uint64_t)dh << 32) | lo; };
+                const unsigned ab = na ? (unsigned)qc % na : 0u;
+                if (na && !mbar_wait(&ctl->a_full[ab], ((unsigned)qc / na) & 1u, status, a.wait_ns)) { ok = false; break; }
+                const uint32_t a_lo = smem_lo + ab * (a.abytes >> 4), half = 16u * (unsigned)ca.kbk;   // 128 rows
                 for (unsigned e = e0; e < e1 && ok; ++e) {
                     unsigned hm = 3u;   // one SM: live 128-row halves of the item's S tile
                     if (!kPair && a.half) {
@@ -488,37 +519,37 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                     if (!got) { ok = false; break; }
                     if (kTimes) w_acc += clock64() - t_a;
                     tc_fence_after();
-                    const unsigned d_tmem = tmem + acc * kTileS;                 // pair: 256 columns
-                    const unsigned d0 = tmem + bh[0] * 128u, d1 = tmem + bh[1] * 128u;   // one SM: 2 x 128
-                    const unsigned bhalf = 16u * (unsigned)ca.kbk;               // 128 B rows, in 16 bytes
+                    if (*(volatile int*)&ctl->abort_flag) { ok = false; break; }
+                    // one SM, both halves live and their accumulators side by side: one MMA over 256 columns
+                    const bool joined = !kPair && hm == 3u && bh[0] < 3u;
                     for (int kb = 0; kb < kblocks; ++kb) {
                         const long long t_o = kTimes ? clock64() : 0;
                         if (!mbar_wait(&ctl->full[stage], phase, status, a.wait_ns)) { ok = false; break; }
                         if (kTimes) w_op += clock64() - t_o;
-                        if (*(volatile int*)&ctl->abort_flag) { ok = false; break; }
                         tc_fence_after();
                         // descriptors: a constant or a half's offset added to the low word of the stage's (built
                         // from pointers, with their conversions, they were most of what the issuing thread did, and
                         // it paced the screen: 70 to 90 % of its time went by outside its waits)
-                        const uint32_t sl = smem_lo + stage * (kStageBytes >> 4);
+                        const uint32_t sl = ring_lo + stage * (stage_bytes >> 4);
+                        const uint32_t al = na ? a_lo + kb * half : sl, bl = na ? sl : sl + (Cfg::kBhi >> 4);
 #pragma unroll
-                        for (int k = 0; k < kBK / 16; ++k) {
-                            if (k >= ksteps) break;
-                            const unsigned accum = (kb | k) != 0 ? 1u : 0u;
-                            const uint64_t ad = desc(sl + 2 * k);
-                            if (kPair) {
-                                umma_f16_pair(d_tmem, ad, desc(sl + (Cfg::kBhi >> 4) + 2 * k), a.idesc_pair, accum);
-                            } else {
+                        for (int h = 0; h < (kPair ? 1 : 2); ++h) {
+                            if (!kPair && (!((hm >> h) & 1u) || (joined && h))) continue;
+                            const unsigned dd = kPair ? tmem + acc * kTileS : tmem + bh[h] * 128u;
+                            const uint32_t bo = bl + (h ? half : 0u);
+                            const unsigned id = kPair ? a.idesc_pair : joined ? a.idesc2 : a.idesc;
 #pragma unroll
-                                for (int h = 0; h < 2; ++h) {
-                                    if (!((hm >> h) & 1u)) continue;
-                                    const unsigned dd = h ? d1 : d0;
-                                    const uint32_t bo = (h ? bhalf : 0u) + 2 * k;
-                                    const uint64_t bd = desc(sl + (Cfg::kBhi >> 4) + bo);
-                                    umma_f16(dd, ad, bd, a.idesc, accum);
+                            for (int k = 0; k < kBK / 16; ++k) {
+                                if (k >= ksteps) break;
+                                const unsigned accum = (kb | k) != 0 ? 1u : 0u;
+                                const uint64_t ad = desc(al + 2 * k), bd = desc(bo + 2 * k);
+                                if (kPair) {
+                                    umma_f16_pair(dd, ad, bd, id, accum);
+                                } else {
+                                    umma_f16(dd, ad, bd, id, accum);
                                     if (kSplit) {   // z.w ~ hi.hi + hi.lo + lo.hi, one FP32 accumulator
-                                        umma_f16(dd, ad, desc(sl + (Cfg::kBlo >> 4) + bo), a.idesc, 1u);
-                                        umma_f16(dd, desc(sl + (Cfg::kAlo >> 4) + 2 * k), bd, a.idesc, 1u);
+                                        umma_f16(dd, ad, desc(bo + ((Cfg::kBlo - Cfg::kBhi) >> 4) + 2 * k), id, 1u);
+                                        umma_f16(dd, desc(al + (Cfg::kAlo >> 4) + 2 * k), bd, id, 1u);
                                     }
                                 }
                             }
@@ -537,6 +568,7 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                     }
                     ++n_mma;
                 }
+                if (na) umma_commit_pair_mc(&ctl->a_empty[ab], 0x3);   // the R tile is free when these MMAs complete
             }
             if (!kPair && n_mma) atomicAdd(&a.ctr->items, n_mma);
             if (!ok) ctl->abort_flag = 1;
@@ -1068,6 +1100,7 @@ void screen_tc(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) {
     a.jps = g.jps;
     a.ncls = g.ncls;
     a.idesc = make_idesc(1u, bf ? 1u : 0u, kTileR, 128u);   // one SM: 128-column half-items
+    a.idesc2 = make_idesc(1u, bf ? 1u : 0u, kTileR, kTileS);   // both halves
     a.idesc_pair = make_idesc(1u, bf ? 1u : 0u, 2 * kTileR, kTileS);
     a.ntR = (unsigned)g.tR[0]->ntiles;
     a.ntS = (unsigned)g.tS[0]->ntiles;
@@ -1086,6 +1119,22 @@ void screen_tc(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) {
     a.cta_t = g.cta_t;
     a.role_t = g.role_t;
     a.nstages = g.stages;
+    if (pair) {
+        // A chunk's R tile stays in shared memory where it leaves room for four stages of S k-blocks (rows of up to
+        // 512 elements; two tiles, the next one brought in early, up to 256).  It halves what the pair reads from
+        // L2: 500,000 x 500,000, d = 512, 204.4 -> 194.8 ms, at the power limit on both sides.  One SM's tile does
+        // not gain: 60,000 rows of 512 leave two stages, whose bytes in flight do not cover the latency (1.74 ->
+        // 1.85 ms), and narrow rows are not bound there (1M x 1M, d = 64, split: 10.15 -> 10.05 ms).
+        const size_t pool = (size_t)StageCfgPair::kStages * StageCfgPair::kBytes;
+        const size_t ab = (size_t)256 * a.cls[0].kpad, sb = (size_t)256 * a.cls[0].kbk;
+        a.na = 2 * ab + 4 * sb <= pool ? 2 : ab + 4 * sb <= pool ? 1 : 0;
+        a.abytes = (unsigned)ab;
+        a.stage_bytes = (unsigned)sb;
+        if (a.na) {
+            const int fit = (int)std::min<size_t>(kMaxRing, (pool - a.na * ab) / sb);
+            a.nstages = g.stages >= 2 ? std::min(g.stages, fit) : fit;
+        }
+    }
     a.half = g.half_packed ? 1 : 0;
     a.njoins = (unsigned)g.njoins;
     TJ_CUDA(cudaMemsetAsync(&eb.ctr->chunk_next, 0, sizeof(unsigned long long), st));
