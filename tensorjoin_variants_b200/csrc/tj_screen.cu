@@ -711,20 +711,22 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                 // stays rolled (one copy of the test in the instruction cache); the per-block masks sit
                 // in a small per-thread array indexed by block.
                 uint32_t cmk[4] = {0u, 0u, 0u, 0u}, imk[4] = {0u, 0u, 0u, 0u};
+                // one SM: 16 columns are read ahead of the 16 under test.  PIPE_FIGURES
+                uint32_t ra[16], rb[16];
+                if (!kPair) tmem_ld16(tbase, ra);
 #pragma unroll 1
                 for (int i = 0; i < 4; ++i) {
                     const int cb = cb_begin + i;
                     if (cb >= cb_end) break;
                     const int col0 = (int)colbase + cb * 32;   // column of the S tile
                     uint32_t raw[32];
-                    tmem_ld32(tbase + cb * 32, raw);
-                    tmem_ld_wait();
-                    if (cb == cb_end - 1) {   // this warp's part read: hand it back
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-                            if (kPair) mbar_arrive_cluster(mapa_shared(&ctl->acc_empty[b], 0));
-                            else mbar_arrive(&ctl->acc_empty[b]);
+                    if (kPair) {
+                        tmem_ld32(tbase + cb * 32, raw);
+                        tmem_ld_wait();
+                        if (cb == cb_end - 1) {   // this warp's part read: hand it back
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster(mapa_shared(&ctl->acc_empty[b], 0));
                         }
                     }
                     uint32_t cm = 0, im = 0;
@@ -770,10 +772,8 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                         // matters where the norms vary inside a group (clustered data); a group that
                         // passes tau sets its bits from the same eight values
                         const float4* nb4 = reinterpret_cast<const float4*>(&m.nrm2f[col0]);
-#pragma unroll
-                        for (int g = 0; g < 4; ++g) {
+                        auto test8 = [&](const uint32_t* r8, int g) {
                             const float4 b0 = nb4[2 * g], b1 = nb4[2 * g + 1];
-                            const uint32_t* r8 = raw + 8 * g;
                             float v[8];
                             fma_m2_x2(__uint_as_float(r8[0]), __uint_as_float(r8[1]), b0.x, b0.y, v[0], v[1]);
                             fma_m2_x2(__uint_as_float(r8[2]), __uint_as_float(r8[3]), b0.z, b0.w, v[2], v[3]);
@@ -787,7 +787,21 @@ __global__ void __launch_bounds__(kScreenThreads, 1)
                                     im |= (v[k] <= tau_in ? 1u : 0u) << (8 * g + k);
                                 }
                             }
+                        };
+                        tmem_wait16(ra);
+                        tmem_ld16(tbase + cb * 32 + 16, rb);
+                        test8(ra, 0);
+                        test8(ra + 8, 1);
+                        tmem_wait16(rb);
+                        if (i < 3) {
+                            tmem_ld16(tbase + cb * 32 + 32, ra);
+                        } else {   // the half-item is read: hand it back
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&ctl->acc_empty[b]);
                         }
+                        test8(rb, 2);
+                        test8(rb + 8, 3);
                     }
                     if (jp.self_join && cm) {   // keep sorted column > sorted row only
                         const int lim = (int)rs - (int)(c0 + col0);   // columns k <= lim: not above the diagonal
