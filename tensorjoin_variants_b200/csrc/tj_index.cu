@@ -632,7 +632,7 @@ __global__ void prep_rows(const void* src, int dtype, long long n, int d, int kp
         float x = xv[u];
         if (!isfinite(x)) { flags |= 1u; x = 0.f; }
         if (kScreen == kScreenPlain) {
-            if (k < d) xs[(size_t)r * d + k] = x;
+            if (k < plain_ld(d)) xs[(size_t)r * plain_ld(d) + k] = x;   // (0 beyond d)
             sx += (double)x * x;
         } else if (kScreen == kScreenInt8Limb) {   // q = 128 h + l, h = floor((q + 64) / 128)
             const int q = (int)x;
@@ -722,8 +722,23 @@ __global__ void prep_rows(const void* src, int dtype, long long n, int d, int kp
     }
 }
 
-// Tile statistics: one block per tile; kL lanes per row (4, 8 or 32), 256 / kL rows at a time.
-template <int kL>
+// kV consecutive elements (4: rows of a multiple of four elements, on a boundary of four)
+template <int kV>
+TJ_DEV void load_xv(const void* src, int dtype, size_t idx, float* v) {
+    if (kV == 1) {
+        v[0] = load_x(src, dtype, idx);
+    } else if (dtype == kF32) {
+        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>((const float*)src + idx);
+    } else {
+        const short4 x = *reinterpret_cast<const short4*>((const int16_t*)src + idx);
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    }
+}
+
+// Tile statistics: one block per tile; kL lanes per row (4, 8 or 32), 256 / kL rows at a time, kV elements per
+// lane and load.  The rows come by permutation, twice (mean and box, then radius), and what bounds the kernel is
+// their bytes in flight: VEC_FIGURES
+template <int kL, int kV>
 __global__ void __launch_bounds__(256) tile_stats_kernel(const void* src, int dtype, long long n, int d, int tile,
                                                          int ntiles, const uint32_t* perm, const double* nrm2,
                                                          const float* nrm2f, const float* zn, const float* en,
@@ -754,31 +769,35 @@ __global__ void __launch_bounds__(256) tile_stats_kernel(const void* src, int dt
             pmin[grp * d + k] = INFINITY;
             pmax[grp * d + k] = -INFINITY;
         }
+        if (kV > 1) __syncwarp();   // a lane's elements below are not those that it has just set
         constexpr int kU = 8;   // rows of a group whose loads are issued together
         for (int i = grp; i < nv; i += kU * kNG) {
             size_t base[kU];
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
                 const int ii = i + u * kNG;
-                base[u] = ii < nv ? (size_t)perm[r0 + ii] * d : 0;
+                base[u] = (size_t)perm[r0 + (ii < nv ? ii : 0)] * d;
             }
-            for (int k = sub; k < d; k += kL) {
-                float v[kU];
+            for (int k = sub * kV; k < d; k += kL * kV) {
+                float v[kU][kV];
 #pragma unroll
-                for (int u = 0; u < kU; ++u) v[u] = i + u * kNG < nv ? load_x(src, dtype, base[u] + k) : 0.f;
-                double sm = psum[grp * d + k];
-                float mn = pmin[grp * d + k], mx = pmax[grp * d + k];
+                for (int u = 0; u < kU; ++u) load_xv<kV>(src, dtype, base[u] + k, v[u]);
 #pragma unroll
-                for (int u = 0; u < kU; ++u) {
-                    if (i + u * kNG < nv) {
-                        sm += v[u];
-                        mn = fminf(mn, v[u]);
-                        mx = fmaxf(mx, v[u]);
+                for (int q = 0; q < kV; ++q) {
+                    double sm = psum[grp * d + k + q];
+                    float mn = pmin[grp * d + k + q], mx = pmax[grp * d + k + q];
+#pragma unroll
+                    for (int u = 0; u < kU; ++u) {
+                        if (i + u * kNG < nv) {
+                            sm += v[u][q];
+                            mn = fminf(mn, v[u][q]);
+                            mx = fmaxf(mx, v[u][q]);
+                        }
                     }
+                    psum[grp * d + k + q] = sm;
+                    pmin[grp * d + k + q] = mn;
+                    pmax[grp * d + k + q] = mx;
                 }
-                psum[grp * d + k] = sm;
-                pmin[grp * d + k] = mn;
-                pmax[grp * d + k] = mx;
             }
         }
         __syncthreads();
@@ -826,18 +845,21 @@ __global__ void __launch_bounds__(256) tile_stats_kernel(const void* src, int dt
         for (int u = 0; u < kRU; ++u) {
             const int i = i0 + u * kNG + (int)(lane / kL);
             ok[u] = i < nv;
-            base[u] = ok[u] ? (size_t)perm[r0 + i] * d : 0;
+            base[u] = (size_t)perm[r0 + (ok[u] ? i : 0)] * d;
             s[u] = 0.0;
         }
-        for (int k = sub; k < d; k += kL) {
-            float v[kRU];
+        for (int k = sub * kV; k < d; k += kL * kV) {
+            float v[kRU][kV];
 #pragma unroll
-            for (int u = 0; u < kRU; ++u) v[u] = ok[u] ? load_x(src, dtype, base[u] + k) : 0.f;
-            const double c = (double)s_ctr[k];
+            for (int u = 0; u < kRU; ++u) load_xv<kV>(src, dtype, base[u] + k, v[u]);
 #pragma unroll
-            for (int u = 0; u < kRU; ++u) {
-                const double df = (double)v[u] - c;
-                if (ok[u]) s[u] += df * df;
+            for (int q = 0; q < kV; ++q) {
+                const double c = (double)s_ctr[k + q];
+#pragma unroll
+                for (int u = 0; u < kRU; ++u) {
+                    const double df = (double)v[u][q] - c;
+                    if (ok[u]) s[u] += df * df;
+                }
             }
         }
 #pragma unroll
@@ -1504,34 +1526,43 @@ TJ_DEV void tile_bounds(const float* sm, const float* ctrT, const float* loT, co
                         int d, float (&ball)[kCandI], float (&box)[kCandI]) {
 #pragma unroll
     for (int ii = 0; ii < kCandI; ++ii) ball[ii] = box[ii] = 0.f;
-#pragma unroll 2
-    for (int k = 0; k < d; ++k) {
-        const float cj = ctrT[(size_t)k * pitch + j];
-        const float lj = loT[(size_t)k * pitch + j];
-        const float hj = hiT[(size_t)k * pitch + j];
-        const float* row = sm + (size_t)k * 3 * kCandI;
-        constexpr int kV = kCandI < 4 ? kCandI : 4;
+    constexpr int kK = kCandI < 16 ? 8 : 2;   // dimensions whose loads are issued together
+    for (int k0 = 0; k0 < d; k0 += kK) {
+        float cj[kK], lj[kK], hj[kK];
 #pragma unroll
-        for (int i0 = 0; i0 < kCandI; i0 += kV) {
-            float c[kV], lo[kV], hi[kV];
-            if (kV == 4) {
-                *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(row + i0);
-                *reinterpret_cast<float4*>(lo) = *reinterpret_cast<const float4*>(row + kCandI + i0);
-                *reinterpret_cast<float4*>(hi) = *reinterpret_cast<const float4*>(row + 2 * kCandI + i0);
-            } else {
+        for (int q = 0; q < kK; ++q) {
+            const size_t at = (size_t)min(k0 + q, d - 1) * pitch + j;
+            cj[q] = ctrT[at];
+            lj[q] = loT[at];
+            hj[q] = hiT[at];
+        }
+#pragma unroll
+        for (int q = 0; q < kK; ++q) {
+            if (k0 + q >= d) break;
+            const float* row = sm + (size_t)(k0 + q) * 3 * kCandI;
+            constexpr int kV = kCandI < 4 ? kCandI : 4;
+#pragma unroll
+            for (int i0 = 0; i0 < kCandI; i0 += kV) {
+                float c[kV], lo[kV], hi[kV];
+                if (kV == 4) {
+                    *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(row + i0);
+                    *reinterpret_cast<float4*>(lo) = *reinterpret_cast<const float4*>(row + kCandI + i0);
+                    *reinterpret_cast<float4*>(hi) = *reinterpret_cast<const float4*>(row + 2 * kCandI + i0);
+                } else {
+#pragma unroll
+                    for (int v = 0; v < kV; ++v) {
+                        c[v] = row[i0 + v];
+                        lo[v] = row[kCandI + i0 + v];
+                        hi[v] = row[2 * kCandI + i0 + v];
+                    }
+                }
 #pragma unroll
                 for (int v = 0; v < kV; ++v) {
-                    c[v] = row[i0 + v];
-                    lo[v] = row[kCandI + i0 + v];
-                    hi[v] = row[2 * kCandI + i0 + v];
+                    const float dc = c[v] - cj[q];
+                    ball[i0 + v] = fmaf(dc, dc, ball[i0 + v]);
+                    const float gap = fmax3(lj[q] - hi[v], lo[v] - hj[q], 0.f);
+                    box[i0 + v] = fmaf(gap, gap, box[i0 + v]);
                 }
-            }
-#pragma unroll
-            for (int v = 0; v < kV; ++v) {
-                const float dc = c[v] - cj;
-                ball[i0 + v] = fmaf(dc, dc, ball[i0 + v]);
-                const float gap = fmax3(lj - hi[v], lo[v] - hj, 0.f);
-                box[i0 + v] = fmaf(gap, gap, box[i0 + v]);
             }
         }
     }
@@ -2061,7 +2092,7 @@ void prepare_side(Side& s, const FrameParams* fpd, bool pca_frame, const float* 
             s.rec = DBuf<I8Row>(rp, st);
         }
     }
-    if (s.screen == kScreenPlain) s.xs = DBuf<float>(rp * s.d, st);
+    if (s.screen == kScreenPlain) s.xs = DBuf<float>(rp * plain_ld(s.d), st);
     s.nrm2 = DBuf<double>(rp, st);
     s.nrm2f = DBuf<float>(rp, st);
     s.zn = DBuf<float>(rp, st);
@@ -2115,9 +2146,11 @@ void tile_stats(const Side& s, int tile, TileSet& ts, cudaStream_t st) {
                tabled ? (const uint32_t*)ts.row0.p : (const uint32_t*)nullptr,
                tabled ? (const uint32_t*)ts.nvalid.p : (const uint32_t*)nullptr, warp_rows);
     };
-    if (L == 4) run(tile_stats_kernel<4>);
-    else if (L == 8) run(tile_stats_kernel<8>);
-    else run(tile_stats_kernel<32>);
+    const bool vec = s.d >= 96 && s.d % 4 == 0 && (uintptr_t)s.src % (s.dtype == kF32 ? 16 : 8) == 0;
+    if (L == 4) run(tile_stats_kernel<4, 1>);
+    else if (L == 8) run(tile_stats_kernel<8, 1>);
+    else if (vec) run(tile_stats_kernel<32, 4>);
+    else run(tile_stats_kernel<32, 1>);
 }
 
 void gather_rows(const std::vector<const void*>& srcs, const std::vector<long long>& rows, int d, int esize,
@@ -2165,7 +2198,11 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
         return;
     }
     DBuf<uint32_t> bitmap((size_t)ntiles * words, st);   // every word is written by the test
-    const int ci = (size_t)3 * 16 * d * sizeof(float) <= 200 * 1024 ? 16 : (size_t)3 * 4 * d * sizeof(float) <= 200 * 1024 ? 4 : 1;
+    // R tiles per block: 16, which read the S tiles' statistics least often, where such blocks fill the device and
+    // their statistics shared memory, else 4.  CAND_FIGURES
+    const size_t row16 = (size_t)3 * 16 * d * sizeof(float);
+    const long long blocks16 = (long long)((ntS + 255) / 256) * ((ntiles + 15) / 16);
+    const int ci = row16 <= 200 * 1024 && blocks16 >= num_sms() ? 16 : row16 / 4 <= 200 * 1024 ? 4 : 1;
     const size_t smem = (size_t)3 * ci * d * sizeof(float);
     if (smem > 200 * 1024) fail(-7, "dimension too large for the candidate test");
     dim3 grid((unsigned)((ntS + 255) / 256), (unsigned)((ntiles + ci - 1) / ci));

@@ -143,6 +143,9 @@ static_assert(sizeof(I8Row) == 16, "a tile's records are one bulk copy");
 __host__ __device__ constexpr int i8_rtiles(int kblocks) { return kblocks == 1 ? 4 : 2; }
 
 // ------------------------------------------------------------------ prepared side (tj_index.cu)
+// Elements from one row to the next in a plain side: 16-byte copies whatever d is.
+__host__ __device__ constexpr int plain_ld(int d) { return (d + 3) & ~3; }
+
 // A side of the join in Morton order: permutation, MMA operand and per-row certificate metadata.
 // Row r of every array is the point perm[r] of the caller's input.
 struct Side {
@@ -163,7 +166,7 @@ struct Side {
     DBuf<uint64_t> keys;         // [n] Morton keys (sorted)
     DBuf<uint16_t> op;           // [rows_pad, kpad or 2*kpad] bf16 / fp16 operand of x - centre
     DBuf<int8_t> op8;            // [rows_pad, 2*kpad] int8 limbs [hi | lo] (int8 limb screen)
-    DBuf<float> xs;              // [rows_pad, d] FP32 rows in sorted order (plain screen)
+    DBuf<float> xs;              // [rows_pad, plain_ld(d)] FP32 rows in sorted order (plain screen)
     DBuf<double> nrm2;           // [rows_pad] sequential FP64 sum of squares of x
     DBuf<float> nrm2f;           // [rows_pad] FP32 nearest of nrm2
     DBuf<float> zn;              // [rows_pad] upper bound of ||z|| (z = operand row)

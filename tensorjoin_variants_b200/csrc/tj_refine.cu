@@ -72,12 +72,12 @@ constexpr int kPStages = 3;
 constexpr int kPRows = kTileR + kPCols; // staged rows: R tile, then the unit's S rows
 
 struct PlainClass {
-    const float* rx;     // [rows, d] FP32 rows (R side of the class)
-    const float* sx;     // [rows, d] FP32 rows (S side)
+    const float* rx;     // [rows, ld] FP32 rows (R side of the class)
+    const float* sx;     // [rows, ld] FP32 rows (S side)
     const uint32_t* r_emit;
     const uint32_t* s_emit;
-    int d;
-    int vec;             // rows are multiples of 16 bytes, 16-byte aligned
+    int d, ld;           // elements of a row, and from one row to the next
+    int vec;             // rows are 16-byte aligned, with zeros up to a multiple of four elements
 };
 
 // Direct joins (kDirect below): every pair of one small join, straight from the caller's rows.
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
             stt = make_uint2(u * kPCols, min((unsigned)kPCols, a.dir.nS - u * kPCols));
             th = a.dir.thr;
             const PlainClass& pc = a.cls[0];
-            pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.d + lq;
-            pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.d + lq;
+            pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.ld + lq;
+            pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.ld + lq;
             if (!(a.dir.upper && stt.x + kPCols <= rt.x + 1)) break;   // (the bitmap of an upper join starts at 0)
             step();
         }
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
                     rt = a.rtiles[I];
                     // rows past a tile's points repeat its last one, so no read leaves the side
                     const PlainClass& pc = a.cls[rt.w];
-                    pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.d + lq;
-                    pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.d + lq;
+                    pr0 = pc.rx + (size_t)(rt.x + min(lr, rt.y - 1)) * pc.ld + lq;
+                    pr1 = pc.rx + (size_t)(rt.x + min(lr + 64, rt.y - 1)) * pc.ld + lq;
                     self_join = a.jps[rt.z].self_join != 0;
                     th = a.thr[rt.z];
                 }
@@ -252,15 +252,26 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         const unsigned c0 = stt.x + p, nvJ = min(stt.y - p, (unsigned)kPCols);
         const PlainClass& pc = a.cls[rt.w];
         const int d = pc.d, kc = min(kPK, d - k0);
-        if (pc.vec) {
-            if (k0 == 0) ps = pc.sx + (size_t)(c0 + min(lr, nvJ - 1)) * d + lq;
+        if (!kDirect || pc.vec) {
+            if (k0 == 0) ps = pc.sx + (size_t)(c0 + min(lr, nvJ - 1)) * pc.ld + lq;
             if ((int)lq < kc) {
                 cp_async16(&sm[buf][lr][lq], pr0 + k0);
                 cp_async16(&sm[buf][lr + 64][lq], pr1 + k0);
                 cp_async16(&sm[buf][kTileR + lr][lq], ps + k0);
             }
+        } else if (kc > kPK / 2) {   // rows of any alignment: element k of every 16th row
+            const int k = threadIdx.x & (kPK - 1), r = threadIdx.x / kPK;
+            const bool real = k < kc;
+            const float* R = pc.rx + (size_t)rt.x * d + k0 + min(k, kc - 1);
+            const float* S = pc.sx + (size_t)c0 * d + k0 + min(k, kc - 1);
+#pragma unroll
+            for (int i = 0; i < kTileR; i += kPT / kPK)
+                cp_async4_zfill(&sm[buf][r + i][k], R + min((unsigned)(r + i), rt.y - 1) * (unsigned)d, real);
+#pragma unroll
+            for (int i = 0; i < kPCols; i += kPT / kPK)
+                cp_async4_zfill(&sm[buf][kTileR + r + i][k], S + min((unsigned)(r + i), nvJ - 1) * (unsigned)d, real);
         } else {   // elements up to the next power of two, zero beyond kc
-            const int lk = kc <= 2 ? 1 : kc <= 4 ? 2 : kc <= 8 ? 3 : 4;
+            const int lk = kc <= 2 ? 1 : kc <= 4 ? 2 : 3;
             for (int idx = threadIdx.x; idx < kPRows << lk; idx += kPT) {
                 const int r = idx >> lk, k = idx & ((1 << lk) - 1);
                 const float* row = r < kTileR ? pc.rx + (size_t)(rt.x + min((unsigned)r, rt.y - 1)) * d
@@ -329,7 +340,6 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         }
         if (!in.last) continue;
         // classify the thread's 32 pairs: bit i * kPJ + j
-        
         float v[kPI * kPJ];
 #pragma unroll
         for (int b = 0; b < kPI * kPJ; ++b) v[b] = sum_x2(acc[b / kPJ][b % kPJ]);
@@ -768,7 +778,7 @@ bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool 
     launch(direct_check, nb, 256, 0, st, R, er, S, es, limit, rows.p, nR, band.p, bad.p);
     PlainArgs a;
     memset(&a, 0, sizeof(a));
-    a.cls[0] = PlainClass{R, S, nullptr, nullptr, jp.d,
+    a.cls[0] = PlainClass{R, S, nullptr, nullptr, jp.d, jp.d,
                           jp.d % 4 == 0 && ((((uintptr_t)R) | ((uintptr_t)S)) & 15) == 0 ? 1 : 0};
     a.dir = DirectArgs{nR, nS, cols64, upper ? 1 : 0, R == S && !upper ? 1 : 0, bits.p, rows.p, band.p, jp.T, fp32_sum_threshold(jp)};
     const unsigned units = (nR + kTileR - 1) / kTileR * cols64;
@@ -802,7 +812,8 @@ void screen_plain(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st) 
         a.cls[c].r_emit = R.emit;
         a.cls[c].s_emit = S.emit;
         a.cls[c].d = R.d;
-        a.cls[c].vec = R.d % 4 == 0 ? 1 : 0;   // the prepared sides are 256-byte aligned
+        a.cls[c].ld = plain_ld(R.d);
+        a.cls[c].vec = 1;
     }
     DBuf<float2> dth((size_t)g.njoins, st);
     fp32_sum_thresholds(g, dth.p, st);
