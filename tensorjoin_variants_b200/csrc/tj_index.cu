@@ -737,7 +737,7 @@ TJ_DEV void load_xv(const void* src, int dtype, size_t idx, float* v) {
 
 // Tile statistics: one block per tile; kL lanes per row (4, 8 or 32), 256 / kL rows at a time, kV elements per
 // lane and load.  The rows come by permutation, twice (mean and box, then radius), and what bounds the kernel is
-// their bytes in flight: VEC_FIGURES
+// their bytes in flight (60,000 x 512, tiles of 128 and of 256 rows: 297 us with kV = 1, 146 with 4)
 template <int kL, int kV>
 __global__ void __launch_bounds__(256) tile_stats_kernel(const void* src, int dtype, long long n, int d, int tile,
                                                          int ntiles, const uint32_t* perm, const double* nrm2,
@@ -1526,46 +1526,57 @@ TJ_DEV void tile_bounds(const float* sm, const float* ctrT, const float* loT, co
                         int d, float (&ball)[kCandI], float (&box)[kCandI]) {
 #pragma unroll
     for (int ii = 0; ii < kCandI; ++ii) ball[ii] = box[ii] = 0.f;
-    constexpr int kK = kCandI < 16 ? 8 : 2;   // dimensions whose loads are issued together
-    for (int k0 = 0; k0 < d; k0 += kK) {
-        float cj[kK], lj[kK], hj[kK];
+    auto add = [&](int k, float cj, float lj, float hj) {
+        const float* row = sm + (size_t)k * 3 * kCandI;
+        constexpr int kV = kCandI < 4 ? kCandI : 4;
+#pragma unroll
+        for (int i0 = 0; i0 < kCandI; i0 += kV) {
+            float c[kV], lo[kV], hi[kV];
+            if (kV == 4) {
+                *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(row + i0);
+                *reinterpret_cast<float4*>(lo) = *reinterpret_cast<const float4*>(row + kCandI + i0);
+                *reinterpret_cast<float4*>(hi) = *reinterpret_cast<const float4*>(row + 2 * kCandI + i0);
+            } else {
+#pragma unroll
+                for (int v = 0; v < kV; ++v) {
+                    c[v] = row[i0 + v];
+                    lo[v] = row[kCandI + i0 + v];
+                    hi[v] = row[2 * kCandI + i0 + v];
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < kV; ++v) {
+                const float dc = c[v] - cj;
+                ball[i0 + v] = fmaf(dc, dc, ball[i0 + v]);
+                const float gap = fmax3(lj - hi[v], lo[v] - hj, 0.f);
+                box[i0 + v] = fmaf(gap, gap, box[i0 + v]);
+            }
+        }
+    };
+    // the loads of the next kK dimensions are under way while these are added up (issued and used in one
+    // iteration, the compiler puts every load next to its use)
+    constexpr int kK = kCandI < 16 ? 8 : 2;
+    float cj[kK], lj[kK], hj[kK];
+    auto load = [&](int k) {
 #pragma unroll
         for (int q = 0; q < kK; ++q) {
-            const size_t at = (size_t)min(k0 + q, d - 1) * pitch + j;
+            const size_t at = (size_t)(k + q) * pitch + j;
             cj[q] = ctrT[at];
             lj[q] = loT[at];
             hj[q] = hiT[at];
         }
+    };
+    int k = 0;
+    if (d >= kK) load(0);
+    for (; k + kK <= d; k += kK) {
+        float c[kK], l[kK], h[kK];
 #pragma unroll
-        for (int q = 0; q < kK; ++q) {
-            if (k0 + q >= d) break;
-            const float* row = sm + (size_t)(k0 + q) * 3 * kCandI;
-            constexpr int kV = kCandI < 4 ? kCandI : 4;
+        for (int q = 0; q < kK; ++q) c[q] = cj[q], l[q] = lj[q], h[q] = hj[q];
+        load(min(k + kK, d - kK));
 #pragma unroll
-            for (int i0 = 0; i0 < kCandI; i0 += kV) {
-                float c[kV], lo[kV], hi[kV];
-                if (kV == 4) {
-                    *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(row + i0);
-                    *reinterpret_cast<float4*>(lo) = *reinterpret_cast<const float4*>(row + kCandI + i0);
-                    *reinterpret_cast<float4*>(hi) = *reinterpret_cast<const float4*>(row + 2 * kCandI + i0);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < kV; ++v) {
-                        c[v] = row[i0 + v];
-                        lo[v] = row[kCandI + i0 + v];
-                        hi[v] = row[2 * kCandI + i0 + v];
-                    }
-                }
-#pragma unroll
-                for (int v = 0; v < kV; ++v) {
-                    const float dc = c[v] - cj[q];
-                    ball[i0 + v] = fmaf(dc, dc, ball[i0 + v]);
-                    const float gap = fmax3(lj[q] - hi[v], lo[v] - hj[q], 0.f);
-                    box[i0 + v] = fmaf(gap, gap, box[i0 + v]);
-                }
-            }
-        }
+        for (int q = 0; q < kK; ++q) add(k + q, c[q], l[q], h[q]);
     }
+    for (; k < d; ++k) add(k, ctrT[(size_t)k * pitch + j], loT[(size_t)k * pitch + j], hiT[(size_t)k * pitch + j]);
 }
 template <int kCandI>
 TJ_DEV void stage_rtiles(float* sm, const float* ctrT, const float* loT, const float* hiT, int ntR, int I0, int nI,
@@ -2199,7 +2210,7 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
     }
     DBuf<uint32_t> bitmap((size_t)ntiles * words, st);   // every word is written by the test
     // R tiles per block: 16, which read the S tiles' statistics least often, where such blocks fill the device and
-    // their statistics shared memory, else 4.  CAND_FIGURES
+    // their statistics shared memory, else 4 (60,000 x 512 self-join: 30 blocks of 16, 261 us; 118 of 4, 65 us)
     const size_t row16 = (size_t)3 * 16 * d * sizeof(float);
     const long long blocks16 = (long long)((ntS + 255) / 256) * ((ntiles + 15) / 16);
     const int ci = row16 <= 200 * 1024 && blocks16 >= num_sms() ? 16 : row16 / 4 <= 200 * 1024 ? 4 : 1;
