@@ -474,8 +474,7 @@ struct RefineArgs {
     unsigned long long acc_cap;
     Counters* ctr;
     const float2* thr;                  // per join FP32-sum thresholds (the FP32 band stage)
-    int is_int;                         // int16 (int14) rows: exact integer distances against T_int
-    long long T_int;
+    long long T_int;                    // int14 rows: exact integer distances against this
 };
 
 // FP32 sum of squared FP32 differences in four FMA chains (tree depth <= d / 4 + 2), the FP32
@@ -506,31 +505,58 @@ TJ_DEV float fp32_d2(const float* x, const float* y, int d) {
 // int64, so no order of the sum can round (the oracle's exact integer predicate).
 TJ_DEV long long exact_d2_i16(const int16_t* x, const int16_t* y, int d) {
     long long acc = 0;
-    if ((d & 7) == 0 && ((((uintptr_t)x) | ((uintptr_t)y)) & 15) == 0) {
-        const int4* x4 = (const int4*)x;
-        const int4* y4 = (const int4*)y;
-        for (int k = 0; k < d / 8; ++k) {
-            const int4 a = __ldg(x4 + k), b = __ldg(y4 + k);
-            const int av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    auto add2 = [&](int a, int b) {   // two elements
+        const int t0 = (int)(short)(a & 0xffff) - (int)(short)(b & 0xffff), t1 = (a >> 16) - (b >> 16);
+        acc += (long long)t0 * t0 + (long long)t1 * t1;
+    };
+    const uintptr_t at = (uintptr_t)x | (uintptr_t)y;
+    int k = 0;
+    if ((at & 15) == 0) {
+        for (; k + 16 <= d; k += 16) {
+            const int4 a0 = __ldg((const int4*)(x + k)), a1 = __ldg((const int4*)(x + k + 8));
+            const int4 b0 = __ldg((const int4*)(y + k)), b1 = __ldg((const int4*)(y + k + 8));
+            add2(a0.x, b0.x), add2(a0.y, b0.y), add2(a0.z, b0.z), add2(a0.w, b0.w);
+            add2(a1.x, b1.x), add2(a1.y, b1.y), add2(a1.z, b1.z), add2(a1.w, b1.w);
+        }
+    }
+    if ((at & 7) == 0) {
+        for (; k + 16 <= d; k += 16) {
+            int2 a[4], b[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int t0 = (int)(short)(av[u] & 0xffff) - (int)(short)(bv[u] & 0xffff);
-                const int t1 = (av[u] >> 16) - (bv[u] >> 16);
-                acc += (long long)t0 * t0 + (long long)t1 * t1;
-            }
+            for (int u = 0; u < 4; ++u) a[u] = __ldg((const int2*)(x + k) + u), b[u] = __ldg((const int2*)(y + k) + u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) add2(a[u].x, b[u].x), add2(a[u].y, b[u].y);
         }
-    } else {
-        for (int k = 0; k < d; ++k) {
-            const int t = (int)__ldg(x + k) - (int)__ldg(y + k);
-            acc += (long long)t * t;
+    }
+    if ((at & 3) == 0) {
+        for (; k + 8 <= d; k += 8) {
+            int a[4], b[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) a[u] = __ldg((const int*)(x + k) + u), b[u] = __ldg((const int*)(y + k) + u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) add2(a[u], b[u]);
         }
+    }
+    for (; k + 4 <= d; k += 4) {
+        int a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = __ldg(x + k + u), b[u] = __ldg(y + k + u);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc += (long long)(a[u] - b[u]) * (a[u] - b[u]);
+    }
+    for (; k < d; ++k) {
+        const int t = (int)__ldg(x + k) - (int)__ldg(y + k);
+        acc += (long long)t * t;
     }
     return acc;
 }
 
 // Band pairs -> accept buffer.  kFp32: each pair is first decided, where it can be, by the
 // certified FP32 sum (the FP32 band stage); only the rest pay the sequential FP64 terminal.
-template <bool kFp32>
+// kInt: int14 rows.  Their own instance: its wider loads want more registers than the FP64 sums, which lose by
+// them (666,000 pairs of a 50,021 x 100 int14 join, rows of 200 bytes read by element: 198 us; by 8 bytes, 78 us;
+// FP32 rows by whole sectors: 1M x 1M mixture 441 -> 519 us, so they keep to 16 bytes at a time).
+template <bool kFp32, bool kInt>
 __global__ void refine_kernel(const RefineArgs a) {
     const unsigned long long n = min(a.ctr->band_reserved, a.band_cap);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -555,7 +581,7 @@ __global__ void refine_kernel(const RefineArgs a) {
                 const uint64_t i = local / (uint64_t)jp.n_cols, j = local - i * (uint64_t)jp.n_cols;
                 if (i >= (uint64_t)jp.n_rows) {   // not a key the screen wrote: flagged, no row is read
                     atomicOr(&a.ctr->status, (unsigned long long)kStatusGuard);
-                } else if (a.is_int) {   // int14 rows: the exact integer predicate decides every pair
+                } else if (kInt) {   // int14 rows: the exact integer predicate decides every pair
                     const int16_t* xi = (const int16_t*)a.rsrc[lo] + (size_t)i * jp.d;
                     const int16_t* yi = (const int16_t*)a.ssrc[lo] + (size_t)j * jp.d;
                     ok = exact_d2_i16(xi, yi, jp.d) <= a.T_int;
@@ -846,16 +872,18 @@ void refine_band(const ScreenInput& g, const EmitBuffers& eb, bool fp32_stage, c
     a.acc_cap = eb.acc_cap;
     a.ctr = eb.ctr;
     a.thr = nullptr;
-    a.is_int = g.R[0]->dtype == kI16 ? 1 : 0;
+    const bool is_int = g.R[0]->dtype == kI16;
     a.T_int = g.T_int;
-    if (a.is_int && g.njoins != 1) fail(-7, "int16 band refinement runs one join at a time");
-    if (fp32_stage && !a.is_int) {
+    if (is_int && g.njoins != 1) fail(-7, "int16 band refinement runs one join at a time");
+    if (is_int) {
+        launch(refine_kernel<false, true>, num_sms() * 8, 256, 0, st, a);
+    } else if (fp32_stage) {
         DBuf<float2> dth((size_t)g.njoins, st);
         fp32_sum_thresholds(g, dth.p, st);
         a.thr = dth.p;
-        launch(refine_kernel<true>, num_sms() * 8, 256, 0, st, a);
+        launch(refine_kernel<true, false>, num_sms() * 8, 256, 0, st, a);
     } else {
-        launch(refine_kernel<false>, num_sms() * 8, 256, 0, st, a);
+        launch(refine_kernel<false, false>, num_sms() * 8, 256, 0, st, a);
     }
 }
 
