@@ -69,7 +69,8 @@ typedef struct tj_index tj_index;
 
 typedef struct tj_options {
     int64_t initial_capacity;   /* accept / band buffer slots for the first attempt (0: library default) */
-    int32_t chunk_items;        /* tile pairs per scheduling chunk (0: 64) */
+    int32_t chunk_items;        /* tile pairs per scheduling chunk (0: the library's choice, 64 but for int14
+                                   joins, whose chunks shrink to 4 where there are few tile pairs) */
     int32_t flags;              /* TJ_FLAG_* bits */
     /* Tile-shape knobs of the 16-bit tensor-core screens (0: the library's choice; the pairs never
      * change): k_block = elements of K per pipeline stage (64, 32 or 16; must divide the padded row

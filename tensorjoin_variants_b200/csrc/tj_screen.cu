@@ -26,12 +26,14 @@
 //
 // Two forms of the same kernel (512 threads, one CTA per SM, persistent over the chunk list):
 //   one SM (kPair = false): an item is a 128-row R tile x 256-row S tile, issued as two 128-column
-//           half-items (M = 128, N = 128 UMMA) into four TMEM accumulators of 128 columns; half-item
+//           half-items (M = 128, N = 128 UMMA; N = 256 where both halves are live and their accumulators
+//           adjacent) into four TMEM accumulators of 128 columns; half-item
 //           s = 2 item + h goes to accumulator s mod 4 and to epilogue group s mod 3, so the three
 //           groups work on different half-items at once and the MMA can run up to two items ahead
 //   CTA pair (kPair = true, cta_group::2, clusters of 2 SMs, dense single joins with rows of
 //           >= 256 elements): an item is a 256 x 256 tile; each CTA loads its 128 A rows and its
-//           128-row half of B, CTA 0 issues M = 256 UMMAs into both CTAs' TMEM (2 accumulators of
+//           128-row half of B (A once per chunk where it fits beside the ring, see screen_tc),
+//           CTA 0 issues M = 256 UMMAs into both CTAs' TMEM (2 accumulators of
 //           256 columns), stage and accumulator barriers are signalled to both CTAs (tcgen05.commit
 //           multicast) and the epilogue warps of both CTAs release accumulators on CTA 0's barrier
 //
