@@ -437,9 +437,8 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         const JoinParams jp = make_params(j.eps2, j.d, 64, 0, j.nR, ncols[0], self);
         const bool half = screen == TJ_SCREEN_FP16 || screen == TJ_SCREEN_FP16X3;
         unsigned long long hdr[5];
-        const bool upper = mode == TJ_MODE_UPPER;
-        if (join_direct((const float*)j.R, (unsigned)j.nR, (const float*)(self ? j.R : j.S), (unsigned)ncols[0], upper,
-                        jp, half ? 30000.f : 0x1p40f, res->rows, res->cols, hdr, st, ev.e[1], ev.e[2])) {
+        if (join_direct((const float*)j.R, (unsigned)j.nR, (const float*)(self ? j.R : j.S), (unsigned)ncols[0],
+                        (Mode)mode, jp, half ? 30000.f : 0x1p40f, res->rows, res->cols, hdr, st, ev.e[1], ev.e[2])) {
             ev.rec(3, st);
             TJ_CUDA(cudaStreamSynchronize(st));
             res->n_all_rows = (uint32_t)j.nR;

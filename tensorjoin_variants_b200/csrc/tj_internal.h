@@ -335,7 +335,7 @@ bool i8_high_limb_screen(const ScreenInput& g);
 // they leave open, the accepted pairs as a bitmap and from it the rows' ends and columns.  False (and
 // nothing made) when an element is not a number within `limit`.  hdr: pairs, longest row, (that flag),
 // pairs decided in FP64 and accepted there.  The events are recorded around the distances.
-bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool upper, const JoinParams& jp, float limit,
+bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, Mode mode, const JoinParams& jp, float limit,
                  DBuf<uint32_t>& rows, DBuf<uint32_t>& cols, unsigned long long (&hdr)[5], cudaStream_t st,
                  cudaEvent_t screen0, cudaEvent_t screen1);
 // FP64 terminal for the band; fp32_stage puts the certified FP32 band stage in front of it.

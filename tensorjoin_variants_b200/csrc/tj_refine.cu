@@ -805,13 +805,15 @@ __global__ void __launch_bounds__(256) direct_emit(const unsigned long long* bit
 
 }  // namespace
 
-bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool upper, const JoinParams& jp, float limit,
+bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, Mode mode, const JoinParams& jp, float limit,
                  DBuf<uint32_t>& rows, DBuf<uint32_t>& cols, unsigned long long (&hdr)[5], cudaStream_t st,
                  cudaEvent_t screen0, cudaEvent_t screen1) {
+    // (R-S sides may share their first row and differ in length: only the mode says that S is R)
+    const bool self = mode != kModeRS, upper = mode == kModeUpper;
     const unsigned cols64 = (nS + kPCols - 1) / kPCols;
     rows = DBuf<uint32_t>::result(nR, st);
     DBuf<unsigned long long> bits((size_t)nR * cols64, st), band(2 + 5, st);
-    const size_t er = (size_t)nR * jp.d, es = R == S ? 0 : (size_t)nS * jp.d;
+    const size_t er = (size_t)nR * jp.d, es = self ? 0 : (size_t)nS * jp.d;
     const unsigned nb = (unsigned)std::min<size_t>((size_t)num_sms() * 2, (er + es + nR + 1023) / 1024);
     DBuf<uint32_t> bad(nb, st);
     if (upper) TJ_CUDA(cudaMemsetAsync(bits.p, 0, bits.bytes(), st));   // units below the diagonal are passed over
@@ -820,7 +822,7 @@ bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, bool 
     memset(&a, 0, sizeof(a));
     a.cls[0] = PlainClass{R, S, nullptr, nullptr, jp.d, jp.d,
                           jp.d % 4 == 0 && ((((uintptr_t)R) | ((uintptr_t)S)) & 15) == 0 ? 1 : 0};
-    a.dir = DirectArgs{nR, nS, cols64, upper ? 1 : 0, R == S && !upper ? 1 : 0, bits.p, rows.p, band.p, jp.T, fp32_sum_threshold(jp)};
+    a.dir = DirectArgs{nR, nS, cols64, upper ? 1 : 0, mode == kModeDirected ? 1 : 0, bits.p, rows.p, band.p, jp.T, fp32_sum_threshold(jp)};
     const unsigned units = (nR + kTileR - 1) / kTileR * cols64;
     cudaEventRecord(screen0, st);
     launch(plain_kernel<true>, std::min(units, (unsigned)num_sms() * 2), kPT, 0, st, a);
