@@ -2239,7 +2239,8 @@ void build_candidates(const TileSet& tr, const TileSet& ts, double Tp, bool self
     exclusive_scan_u32(c.cnt.p, c.off.p, (size_t)ntR, c.dev_counts.p, sws.p, st);
     launch(cand_fill, (unsigned)((ntR * 32 + 255) / 256), 256, 0, st, bitmap.p, words, ntiles, step, c.off.p, c.jlist.p,
            (const uint32_t*)nullptr);
-    launch(place_chunks, dim3((unsigned)((ntS + chunk_items - 1) / chunk_items), (unsigned)((ntR + kPlaceLists - 1) / kPlaceLists)), 1024,
+    // (size_t: chunk_items may be anything up to 2^31 - 1)
+    launch(place_chunks, dim3((unsigned)(((size_t)ntS + chunk_items - 1) / chunk_items), (unsigned)((ntR + kPlaceLists - 1) / kPlaceLists)), 1024,
            0, st, (const uint32_t*)c.cnt.p, (const uint32_t*)c.off.p, ntR, (unsigned)chunk_items, c.chunks.p,
            c.dev_counts.p + 1);
     TJ_CUDA(cudaGetLastError());
