@@ -322,7 +322,8 @@ void check_status(unsigned long long status) {
     if (status & kStatusBadInput) fail(TJ_ERR_INPUT, "input contains NaN/Inf or a row norm beyond 2^50");
     if (status & kStatusFp16Range) fail(TJ_ERR_RANGE, "input magnitude exceeds the FP16 range; use the BF16 screen");
     if (status & kStatusTmemAlloc) fail(TJ_ERR_CUDA, "tensor memory allocation failed");
-    if (status & kStatusGuard) fail(TJ_ERR_CUDA, "a guard region after an output buffer was overwritten");
+    if (status & kStatusGuard)
+        fail(TJ_ERR_CUDA, "a guard region after an output buffer was overwritten, or a pair key names no row");
 }
 
 struct JoinIn {
@@ -1011,9 +1012,9 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         res->d_cols = std::move(d_cols);
     }
     ev.rec(5, st);
+    // what the ordering found (a key outside the rows, a look-back that gave up, an overwritten guard)
     unsigned long long status_after = 0;
-    if (guards)
-        TJ_CUDA(cudaMemcpyAsync(&status_after, &ctr.p->status, 8, cudaMemcpyDeviceToHost, st));
+    TJ_CUDA(cudaMemcpyAsync(&status_after, &ctr.p->status, 8, cudaMemcpyDeviceToHost, st));
     TJ_CUDA(cudaStreamSynchronize(st));
     check_status(status_after);
     res->count = nvalid;
