@@ -363,9 +363,10 @@ bool direct_join_fits(const JoinIn& j, int mode, const tj_options* opt) {
 
 // One or many joins.  Joins are grouped into classes of equal d; each class gets one
 // concatenated, Morton-sorted side per operand (joins stay contiguous), global tile tables, one
-// block-diagonal candidate list and one persistent screen launch over all classes.
+// block-diagonal candidate list and one persistent screen launch over all classes.  `lean`: with as little
+// memory as the join can do with (the accept buffer starts small, the output is ordered in place).
 void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int screen, const tj_options* opt,
-                    tj_result* res, cudaStream_t st) {
+                    bool lean, tj_result* res, cudaStream_t st) {
     const bool self = mode != TJ_MODE_RS;
     const int nj = (int)joins.size();
     if (nj < 1) fail(TJ_ERR_INVALID, "no joins");
@@ -430,7 +431,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     stage_reset();
     Events ev;
     ev.rec(0, st);
-    if (nj == 1 && !i8 && direct_join_fits(joins[0], mode, opt)) {
+    if (nj == 1 && !i8 && !lean && direct_join_fits(joins[0], mode, opt)) {
         // A small join: all pairs at once, without an index.  Elements beyond what every screen takes (FP16
         // operands: 65504 after centring, so 30000 before) go through the screen that was asked for, which
         // accepts or refuses them.
@@ -800,7 +801,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
                                                                                                    cap / (nj == 1 ? 1 : 8));
     // the accept buffer is temporary, so it starts at 2^25 slots (256 MB) wherever the joins hold that
     // many pairs: 280 neighbours per row of a 100,000-row set ran the whole screen a second time
-    if (!(opt && opt->initial_capacity > 0))
+    if (!(opt && opt->initial_capacity > 0) && !lean)
         cap = std::max(cap, std::min(1ull << 25, (unsigned long long)S_.pairs_all));
     const bool guards = opt && (opt->flags & TJ_FLAG_GUARDS);
     const bool stage_keys = opt && (opt->flags & TJ_FLAG_STAGE_KEYS);
@@ -819,7 +820,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     // pairs per row, then the rows' first positions (counted with every attempt, before the read-back, so
     // that the output can be sized and its form chosen without another wait)
     const bool directed = mode == TJ_MODE_DIRECTED;
-    const bool by_rows = all_rows < 0xFFFFFFFEull;
+    const bool by_rows = all_rows < 0xFFFFFFFEull && !lean;
     const uint32_t nrows = by_rows ? (uint32_t)all_rows : 0u;
     const size_t guard32 = 2 * gs, rows_even = ((size_t)nrows + 1) & ~(size_t)1;
     DBuf<uint32_t> rows, rows_ws;
@@ -1027,11 +1028,24 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     S_.ms_total = ev.ms(0, 5);
 }
 
-// One join (or batch) with its temporaries in the calling thread's workspace.
+// One join (or batch) with its temporaries in the calling thread's workspace.  Where the device has no
+// room for it (the accept buffer alone starts at up to 256 MB), the idle memory held here is given back and
+// the join is done once more with little.
 void run_batch(const std::vector<JoinIn>& joins, int dtype, int mode, int screen, const tj_options* opt,
                tj_result* res, cudaStream_t st) {
+    try {
+        WorkspaceScope ws(st);
+        run_batch_body(joins, dtype, mode, screen, opt, false, res, st);
+        return;
+    } catch (const Error& e) {
+        if (e.code != TJ_ERR_NOMEM) throw;
+    }
+    *res = tj_result();
+    release_cached(st);
+    TJ_CUDA(cudaStreamSynchronize(st));
+    TJ_CUDA(cudaMemPoolTrimTo(pool_for_current(), 0));
     WorkspaceScope ws(st);
-    run_batch_body(joins, dtype, mode, screen, opt, res, st);
+    run_batch_body(joins, dtype, mode, screen, opt, true, res, st);
 }
 
 }  // namespace
