@@ -348,17 +348,21 @@ void check_flags(const tj_options* opt) {
 }
 
 // Joins that are done directly, without an index: no options (every knob is one of the indexed path) and
-// rows of at most 192 elements (longer ones belong to the CTA-pair screen).  The direct path takes 75 us
-// plus about 0.1 ps per pair and element (8 more elements per pair for its classification); the indexed
-// path's forty launches and two waits take 350 to 700 us however small the join.  The line lies at 2^31,
-// 300 us, below the smallest figure measured for the indexed path on the same joins (one B200, whole
-// call, direct | indexed): 311 x 256 x 8 80 | 419 us; 5,003 x 3,217 x 65 214 | 584; 10,000 x 2 directed 184 |
-// 421; 8,000 x 16 upper 154 | 448; 8,000 x 8,000 x 32 291 | 654; beyond it 20,000 x 2 directed 508 | 454.
+// rows of at most 192 elements (longer ones were not measured).  The direct pass takes 75 us plus about
+// 0.1 ps per pair and element (8 more elements per pair for its classification), and it computes whole
+// tiles of 128 R rows; the indexed path's forty launches and two waits take 350 to 700 us however small the
+// join, more with many rows to put in order.  The line lies at 2^31, 300 us, and for sides of few R rows, where
+// S is long, at 2^32 with whole tiles counted.  Whole call, one B200, direct | indexed: 311 x 256 x 8 80 | 419
+// us; 5,003 x 3,217 x 65 214 | 584; 8,000 x 16 upper 154 | 448; 8,000 x 8,000 x 32 291 | 654.  On the line the
+// direct pass wins least against rows in tight clusters, of which the index leaves next to nothing:
+// 20,724 x 2 upper 474 | 508, 18,918 x 4 upper 407 | 448, 7,237 x 33 directed 307 | 383; beyond it 20,000 x 2
+// directed 508 | 454, and 1 x 262,144 x 192 (whole tiles: 1.6 times the line) 2,786 | 931 when it was done directly.
 bool direct_join_fits(const JoinIn& j, int mode, const tj_options* opt) {
     if (opt && (opt->initial_capacity || opt->chunk_items || opt->flags || opt->k_block || opt->stages)) return false;
     const long long nS = mode == TJ_MODE_RS ? j.nS : j.nR;
     if (j.d > 192 || j.nR < 1 || nS < 1 || j.nR > (1ll << 15) || nS > (1ll << 20)) return false;
-    return (double)j.nR * (double)nS / (mode == TJ_MODE_UPPER ? 2 : 1) * (j.d + 8) <= 0x1p31;
+    const double each = (double)nS / (mode == TJ_MODE_UPPER ? 2 : 1) * (j.d + 8);   // work per R row
+    return (double)j.nR * each <= 0x1p31 && (double)((j.nR + kTileR - 1) / kTileR * kTileR) * each <= 0x1p32;
 }
 
 // One or many joins.  Joins are grouped into classes of equal d; each class gets one

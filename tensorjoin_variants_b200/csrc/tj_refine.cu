@@ -116,6 +116,10 @@ TJ_DEV void cp_async4_zfill(void* dst, const void* src, bool real) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
                  :: "r"(smem_u32(dst)), "l"((uint64_t)src), "r"(real ? 4u : 0u) : "memory");
 }
+TJ_DEV void cp_async16_zfill(void* dst, const void* src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 :: "r"(smem_u32(dst)), "l"((uint64_t)src), "r"(real ? 16u : 0u) : "memory");
+}
 // acc += (r - s)^2 in both halves, each rounded as the scalar subtract and fmaf
 TJ_DEV void sqdiff_x2(unsigned long long r, unsigned long long s, unsigned long long& acc) {
     asm("{\n\t.reg .b64 t;\n\t"
@@ -155,7 +159,10 @@ TJ_DEV int find_rtile(const uint32_t* off, int n, uint32_t e) {
 // accepted pairs go to a bitmap instead of the emit buffers, and the few pairs the FP32 sum cannot decide
 // are decided by the thread that finds them, in FP64 from the rows.  Of an upper join only the units with a
 // pair above the diagonal (2 I and later of tile I) are counted, so that every CTA gets as many of them
-// (dealt out with the others, some CTAs had none and some twice the mean: 18,918 x 4 423 -> 321 us, 4,634 x 192 461 -> 293).
+// (dealt out with the others, some CTAs had none and some twice the mean: 18,918 x 4 423 -> 321 us, 4,634 x 192
+// 461 -> 293).  R rows past the last one are zeros in shared memory and nothing else:
+// as copies of it they sent every CTA to the same few lines of L2 (one row against 262,144 x 64: 1,284 us
+// against 209 for 128 rows).
 template <bool kDirect>
 __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
     __shared__ __align__(16) float sm[kPStages][kPRows][kPLd];
@@ -276,8 +283,13 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         if (!kDirect || pc.vec) {
             if (k0 == 0) ps = pc.sx + (size_t)(c0 + min(lr, nvJ - 1)) * pc.ld + lq;
             if ((int)lq < kc) {
-                cp_async16(&sm[buf][lr][lq], pr0 + k0);
-                cp_async16(&sm[buf][lr + 64][lq], pr1 + k0);
+                if (kDirect) {
+                    cp_async16_zfill(&sm[buf][lr][lq], pr0 + k0, lr < rt.y);
+                    cp_async16_zfill(&sm[buf][lr + 64][lq], pr1 + k0, lr + 64 < rt.y);
+                } else {
+                    cp_async16(&sm[buf][lr][lq], pr0 + k0);
+                    cp_async16(&sm[buf][lr + 64][lq], pr1 + k0);
+                }
                 cp_async16(&sm[buf][kTileR + lr][lq], ps + k0);
             }
         } else if (kc > kPK / 2) {   // rows of any alignment: element k of every 16th row
@@ -287,7 +299,8 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
             const float* S = pc.sx + (size_t)c0 * d + k0 + min(k, kc - 1);
 #pragma unroll
             for (int i = 0; i < kTileR; i += kPT / kPK)
-                cp_async4_zfill(&sm[buf][r + i][k], R + min((unsigned)(r + i), rt.y - 1) * (unsigned)d, real);
+                cp_async4_zfill(&sm[buf][r + i][k], R + min((unsigned)(r + i), rt.y - 1) * (unsigned)d,
+                                real && (unsigned)(r + i) < rt.y);
 #pragma unroll
             for (int i = 0; i < kPCols; i += kPT / kPK)
                 cp_async4_zfill(&sm[buf][kTileR + r + i][k], S + min((unsigned)(r + i), nvJ - 1) * (unsigned)d, real);
@@ -297,7 +310,7 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
                 const int r = idx >> lk, k = idx & ((1 << lk) - 1);
                 const float* row = r < kTileR ? pc.rx + (size_t)(rt.x + min((unsigned)r, rt.y - 1)) * d
                                               : pc.sx + (size_t)(c0 + min((unsigned)(r - kTileR), nvJ - 1)) * d;
-                cp_async4_zfill(&sm[buf][r][k], row + k0 + min(k, kc - 1), k < kc);
+                cp_async4_zfill(&sm[buf][r][k], row + k0 + min(k, kc - 1), k < kc && (r >= kTileR || (unsigned)r < rt.y));
             }
         }
         if (threadIdx.x == 0)
@@ -368,7 +381,10 @@ __global__ void __launch_bounds__(kPT, 2) plain_kernel(const PlainArgs a) {
         // rows that hold a near pair in some lane, and only their pairs one by one
         float rm[kPI];
 #pragma unroll
-        for (int i = 0; i < kPI; ++i) rm[i] = fminf(fmin3(v[i * kPJ], v[i * kPJ + 1], v[i * kPJ + 2]), v[i * kPJ + 3]);
+        for (int i = 0; i < kPI; ++i) {
+            rm[i] = fminf(fmin3(v[i * kPJ], v[i * kPJ + 1], v[i * kPJ + 2]), v[i * kPJ + 3]);
+            if (kDirect && (unsigned)(i * 16 + ty) >= in.nvI) rm[i] = INFINITY;   // (no row: zeros)
+        }
         const float m = fmin3(fmin3(rm[0], rm[1], rm[2]), fmin3(rm[3], rm[4], rm[5]), fminf(rm[6], rm[7]));
         const bool near = __any_sync(0xffffffffu, !(m > in.th.y));
         if (!kDirect && !near) continue;
