@@ -273,6 +273,7 @@ struct tj_result {
     // cols, rows of all joins in order), or, with rows.p null, sorted canonical keys (first `count` valid)
     DBuf<uint32_t> rows, cols;
     uint32_t n_all_rows = 0;
+    unsigned long long longest_row = 0;
     RowTables tabs;
     DBuf<RowTable> d_tab;              // batches: the tables' device arrays
     DBuf<unsigned long long> d_rowoff;
@@ -288,6 +289,7 @@ struct tj_result {
     std::vector<int64_t> offsets;
     DBuf<unsigned long long> d_keyoff;
     DBuf<long long> d_cols;
+    RowsView view() const { return RowsView{rows.p, cols.p, n_all_rows, count, longest_row, &tabs}; }
 };
 
 struct tj_index {
@@ -448,6 +450,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
             ev.rec(3, st);
             TJ_CUDA(cudaStreamSynchronize(st));
             res->n_all_rows = (uint32_t)j.nR;
+            res->longest_row = hdr[1];
             res->tabs.first = make_row_table(0, 0, (unsigned long long)ncols[0]);
             res->count = (long long)hdr[0];
             // counts as of a screen over all tile pairs; a directed join's are those of its i < j pairs
@@ -972,6 +975,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         res->rows = std::move(rows);
         res->cols = std::move(cols);
         res->n_all_rows = nrows;
+        res->longest_row = h.longest_row;
     } else {
         rows.reset();
         DBuf<uint64_t> keys;
@@ -1089,7 +1093,7 @@ int tj_result_pairs(const tj_result* res, int64_t* i_out, int64_t* j_out, void* 
     if (!i_out || !j_out) fail(TJ_ERR_INVALID, "null output");
     if (res->njoins > 1) fail(TJ_ERR_INVALID, "batched result: use tj_batch_pairs");
     if (res->rows.p)
-        rows_pairs(res->rows.p, res->cols.p, res->n_all_rows, res->tabs, i_out, j_out, (cudaStream_t)stream);
+        rows_pairs(res->view(), i_out, j_out, (cudaStream_t)stream);
     else
         decode_pairs(res->keys.p, res->count, res->n_cols, i_out, j_out, (cudaStream_t)stream);
     return TJ_OK;
@@ -1102,7 +1106,7 @@ int tj_result_keys(const tj_result* res, uint64_t* keys_out, void* stream) {
     if (res->count == 0) return TJ_OK;
     if (!keys_out) fail(TJ_ERR_INVALID, "null output");
     if (res->rows.p) {
-        rows_keys(res->rows.p, res->cols.p, res->n_all_rows, res->tabs, keys_out, (cudaStream_t)stream);
+        rows_keys(res->view(), keys_out, (cudaStream_t)stream);
         return TJ_OK;
     }
     TJ_CUDA(cudaMemcpyAsync(keys_out, res->keys.p, (size_t)res->count * 8, cudaMemcpyDeviceToDevice,
@@ -1130,7 +1134,7 @@ int tj_result_neighbor_table(const tj_result* res, uint32_t* counts_out, int64_t
     if (res->njoins > 1) fail(TJ_ERR_INVALID, "batched result: not supported");
     cudaStream_t st = (cudaStream_t)stream;
     if (res->rows.p) {
-        rows_neighbors(res->rows.p, res->cols.p, res->n_all_rows, counts_out, res->count > 0 ? flat_out : nullptr, st);
+        rows_neighbors(res->view(), counts_out, res->count > 0 ? flat_out : nullptr, st);
         return TJ_OK;
     }
     TJ_CUDA(cudaMemsetAsync(counts_out, 0, (size_t)res->n_rows * 4, st));
@@ -1264,7 +1268,7 @@ int tj_batch_pairs(const tj_result* res, int64_t* i_out, int64_t* j_out, void* s
     if (res->count == 0) return TJ_OK;
     if (!i_out || !j_out) fail(TJ_ERR_INVALID, "null output");
     if (res->rows.p) {
-        rows_pairs(res->rows.p, res->cols.p, res->n_all_rows, res->tabs, i_out, j_out, (cudaStream_t)stream);
+        rows_pairs(res->view(), i_out, j_out, (cudaStream_t)stream);
         return TJ_OK;
     }
     if (res->njoins == 1) {

@@ -372,12 +372,16 @@ void count_rows(const uint64_t* keys, const Counters* ctr, unsigned long long ca
 void order_rows(const uint64_t* keys, unsigned long long slots, const RowTables& t, bool directed, uint32_t nrows,
                 uint32_t total, unsigned long long longest, uint32_t* cursor, uint32_t* cols,
                 unsigned long long* status, cudaStream_t st);
-void rows_pairs(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, const RowTables& t, int64_t* i_out,
-                int64_t* j_out, cudaStream_t st);
-void rows_keys(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, const RowTables& t, uint64_t* out,
-               cudaStream_t st);
-void rows_neighbors(const uint32_t* row_end, const uint32_t* cols, uint32_t nrows, uint32_t* counts, int64_t* flat,
-                    cudaStream_t st);
+struct RowsView {           // a result by rows
+    const uint32_t *row_end, *cols;
+    uint32_t nrows;
+    long long total;               // pairs, at least one (rows_neighbors: or none, and no flat list)
+    unsigned long long longest;    // most pairs of one row
+    const RowTables* tabs;
+};
+void rows_pairs(const RowsView& v, int64_t* i_out, int64_t* j_out, cudaStream_t st);
+void rows_keys(const RowsView& v, uint64_t* out, cudaStream_t st);
+void rows_neighbors(const RowsView& v, uint32_t* counts, int64_t* flat, cudaStream_t st);
 void rows_batch_offsets(const uint32_t* row_end, const unsigned long long* row_off, int njoins, long long n,
                         long long* out, cudaStream_t st);
 

@@ -809,16 +809,33 @@ __global__ void __launch_bounds__(1024) direct_scan(uint32_t* cnt, unsigned nR, 
     }
 }
 
-// Columns of every row in order, from the bitmap: a warp per row, 32 words at a time.
+// Columns of every row in order, from the bitmap, 32 words at a time: kW = 1 warp per row, or a block, its
+// warps on consecutive parts of the words (rows of kEmitWords words and more, where there are too few of them
+// to fill the device: 16 dense rows of 2^20 columns 13.4 -> 11.0 ms in all).
+constexpr unsigned kEmitWords = 512;
+template <int kW>
 __global__ void __launch_bounds__(256) direct_emit(const unsigned long long* bits, unsigned nR, unsigned cols64,
                                                    const uint32_t* row_end, uint32_t* cols) {
-    const unsigned row = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = lane_id();
-    if (row >= nR) return;   // warp-uniform
+    const unsigned row = (blockIdx.x * 256 + threadIdx.x) / (32 * kW), lane = lane_id(), warp = threadIdx.x >> 5;
+    if (row >= nR) return;   // uniform over the row's warps
     uint32_t pos = row ? row_end[row - 1] : 0u;
     const uint32_t end = row_end[row];
-    for (unsigned u0 = 0; u0 < cols64 && pos < end; u0 += 32) {
+    unsigned first = 0, last = cols64;   // this warp's words
+    if (kW > 1) {
+        __shared__ unsigned before[kW];
+        const unsigned part = (cols64 + kW - 1) / kW;
+        first = min(warp * part, cols64);
+        last = min(first + part, cols64);
+        unsigned n = 0;
+        for (unsigned u = first + lane; u < last; u += 32) n += (unsigned)__popcll(bits[(size_t)row * cols64 + u]);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) before[warp] = n;
+        __syncthreads();
+        for (unsigned w = 0; w < warp; ++w) pos += before[w];
+    }
+    for (unsigned u0 = first; u0 < last && pos < end; u0 += 32) {
         const unsigned u = u0 + lane;
-        unsigned long long w = u < cols64 ? bits[(size_t)row * cols64 + u] : 0ull;
+        unsigned long long w = u < last ? bits[(size_t)row * cols64 + u] : 0ull;
         unsigned tot;
         uint32_t p = pos + warp_excl_scan((unsigned)__popcll(w), tot);
         for (; w; w &= w - 1) cols[p++] = u * 64 + (unsigned)__ffsll((long long)w) - 1;
@@ -859,8 +876,11 @@ bool join_direct(const float* R, unsigned nR, const float* S, unsigned nS, Mode 
         return false;
     }
     cols = DBuf<uint32_t>::result(std::max<size_t>((size_t)hdr[0], 1), st);
-    if (hdr[0])
-        launch(direct_emit, (nR + 7) / 8, 256, 0, st, (const unsigned long long*)bits.p, nR, cols64,
+    if (hdr[0] && cols64 >= kEmitWords && nR <= (unsigned)num_sms() * 8)
+        launch(direct_emit<8>, nR, 256, 0, st, (const unsigned long long*)bits.p, nR, cols64, (const uint32_t*)rows.p,
+               cols.p);
+    else if (hdr[0])
+        launch(direct_emit<1>, (nR + 7) / 8, 256, 0, st, (const unsigned long long*)bits.p, nR, cols64,
                (const uint32_t*)rows.p, cols.p);
     return true;
 }
