@@ -200,9 +200,12 @@ __global__ void neighbor_counts(const uint64_t* keys, long long n, long long n_c
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const uint64_t k = keys[t];
-    const uint64_t i = k / (uint64_t)n_cols;
-    atomicAdd(&counts[i], 1u);
-    if (flat) flat[t] = (int64_t)(k - i * (uint64_t)n_cols);
+    const uint64_t i = k / (uint64_t)n_cols, first = i * (uint64_t)n_cols;
+    // the row's end minus its start, modulo 2^32: two atomics per row (one per pair, on few addresses, was
+    // most of the time: 107M pairs of 30,000 rows 36.5 -> 5.1 ms with the join)
+    if (t == 0 || keys[t - 1] < first) atomicAdd(&counts[i], 0u - (uint32_t)t);
+    if (t == n - 1 || keys[t + 1] >= first + (uint64_t)n_cols) atomicAdd(&counts[i], (uint32_t)t + 1u);
+    if (flat) flat[t] = (int64_t)(k - first);
 }
 
 int bits_for(unsigned long long max_value) {
@@ -864,7 +867,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         ev.rec(4, st);
         if (by_rows) {
             if (guards) launch(guard_fill, 1, 256, 0, st, (uint64_t*)(rows.p + rows_even));
-            count_rows(acc.p, ctr.p, cap, tabs, directed, nrows, rows.p, rows.p, &ctr.p->longest_row, rows_ws.p, st);
+            count_rows(acc.p, ctr.p, cap, tabs, directed, nrows, rows.p, rows.p, rows_ws.p, st);
         }
         if (guards) {
             launch(guard_check, 1, 256, 0, st, (const uint64_t*)(acc.p + cap), ctr.p);
@@ -951,15 +954,18 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     }
     band.reset();
 
-    // canonical order: by rows where no row is longer than a block can sort and the rows are not many
-    // more than the pairs (4 bytes per row and per pair), else by sorting whole keys.  Measured with the
-    // reading of the result (one B200, keys -> rows): 377M pairs of 23.6M rows (2,048 joins) 18.3 -> 12.0
-    // ms; 16.3M pairs of 1M rows 0.76 -> 0.52 ms; 27.5M directed pairs of 100,000 rows as a neighbour
-    // table 2.74 -> 1.06 ms.
+    // canonical order: by rows where they are not many more than the pairs (4 bytes per row and per pair)
+    // and at most half of the pairs lie in rows of more than kMidRow, which a block sorts in shared memory at
+    // up to twice the cost of the whole-key sort; else by sorting whole keys.  Measured with the reading of
+    // the result (one B200, keys -> rows): 377M pairs of 23.6M rows (2,048 joins) 18.3 -> 12.0 ms; 16.3M pairs
+    // of 1M rows 0.76 -> 0.52 ms; 27.5M directed pairs of 100,000 rows as a neighbour table 2.74 -> 1.06 ms.
+    // Whole joins by the share of pairs in long rows, keys | rows: 100,000 x 2 upper, 0.46 2.41 | 2.41 ms; 0.72
+    // 4.23 | 4.62; 30,000 x 2 directed, 0.68 1.30 | 1.42; 0.94 1.85 | 2.40; 1.0 (3,600 a row) 6.8 | 9.9.
     unsigned long long slots = h.acc_reserved;
     long long nvalid = (long long)h.acc_valid + (directed ? (long long)h.acc_valid + joins[0].nR : 0);
-    const bool rows_form = by_rows && nvalid < 0xFFFFFFFFll && slots < 0xFFFFFFFFull && h.longest_row <= kLongRow &&
-                           all_rows <= std::max(2ull * (unsigned long long)nvalid, 1ull << 20);
+    const bool rows_form = by_rows && nvalid < 0xFFFFFFFFll && slots < 0xFFFFFFFFull &&
+                           rows_may_fit((unsigned long long)nvalid, all_rows) && h.longest_row <= kLongRow &&
+                           (nvalid <= (1ll << 20) || 2 * h.long_pairs <= (unsigned long long)nvalid);
     if (rows_form) {
         const size_t cols_even = ((size_t)nvalid + 1) & ~(size_t)1;
         DBuf<uint32_t> cols = DBuf<uint32_t>::result(std::max<size_t>(cols_even, 2) + guard32, st);

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #define TJ_DEV __device__ __forceinline__
@@ -42,6 +43,7 @@ struct Counters {
     unsigned long long band_fp64;      // band pairs that reached the FP64 terminal
     unsigned long long xl_items;       // int8 four-product screen: items that took the low-limb products
     unsigned long long longest_row;    // most pairs of one row (canonical output by rows)
+    unsigned long long long_pairs;     // pairs in rows of more than kMidRow
     unsigned long long status;         // kStatus* bits
     unsigned long long pairs_screened; // distance evaluations of the candidate list
     unsigned long long screen_ops;     // algorithmic screen operations of the candidate list
@@ -49,7 +51,7 @@ struct Counters {
     unsigned long long screen_reserved;  // acc_reserved after the screen, before the refinement appends
     unsigned long long chunk_next;       // work queue of the one-SM screen: chunks taken beyond the first wave
 };
-constexpr int kCountersPerAttempt = 11;
+constexpr int kCountersPerAttempt = (int)(offsetof(Counters, status) / 8);
 
 // Per-join parameters (batched mode has one per join; a single join uses one entry).
 struct JoinParams {

@@ -102,9 +102,11 @@ void stage_reset();
 
 // ------------------------------------------------------------------ scan / sort (tj_sort.cu)
 size_t scan_workspace_elems(size_t n);
-// with `longest` (device, u64) the largest element is raised into it
+// with `lengths` (device, two u64) the largest element is raised into the first, and the sum of the elements
+// above kMidRow added to the second
+constexpr unsigned kMidRow = 512;
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
-                        cudaStream_t st, unsigned long long* longest = nullptr);
+                        cudaStream_t st, unsigned long long* lengths = nullptr);
 size_t radix_workspace_elems(size_t n);   // without a status word
 size_t sweep_workspace_elems(size_t n);   // with one
 // Sorts each segment [off[k], off[k + 1]) (off null: [0, n)) of at most kSegmentSort keys by the low 32
@@ -362,12 +364,17 @@ struct RowTables {
     const unsigned long long* row_off = nullptr;
 };
 RowTable make_row_table(unsigned long long key_off, unsigned long long row_off, unsigned long long n_cols);
-constexpr unsigned long long kLongRow = 16384;         // longest row order_rows sorts
-// Counts the pairs of every row (device slot count, at most cap) and scans the counts: first[r] is row
-// r's first position; *longest is raised to the largest count.  cnt and first may be one array.
-void count_rows(const uint64_t* keys, const Counters* ctr, unsigned long long cap, const RowTables& t, bool directed,
-                uint32_t nrows, uint32_t* cnt, uint32_t* first, unsigned long long* longest, uint32_t* ws,
-                cudaStream_t st);
+constexpr unsigned long long kLongRow = 4096;          // longest row order_rows sorts
+// Whether the output may be ordered by rows, by what is known before the rows are counted: they are not many
+// more than the pairs (four bytes per row and per pair), nor so long that most pairs lie in long ones.
+__host__ __device__ inline bool rows_may_fit(unsigned long long pairs, unsigned long long rows) {
+    return (pairs <= (1ull << 20) || pairs <= 768 * rows) && (rows <= (1ull << 20) || rows <= 2 * pairs);
+}
+// Counts the pairs of every row (device counters, slots up to cap) and scans the counts: first[r] is row
+// r's first position; ctr->longest_row and long_pairs get the rows' lengths.  cnt and first may be one
+// array.  Does nothing where the slots overflowed or the pairs do not fit the form by rows.
+void count_rows(const uint64_t* keys, Counters* ctr, unsigned long long cap, const RowTables& t, bool directed,
+                uint32_t nrows, uint32_t* cnt, uint32_t* first, uint32_t* ws, cudaStream_t st);
 // Puts the columns of the keys in canonical order; `cursor` (first positions) ends as the rows' ends.
 void order_rows(const uint64_t* keys, unsigned long long slots, const RowTables& t, bool directed, uint32_t nrows,
                 uint32_t total, unsigned long long longest, uint32_t* cursor, uint32_t* cols,

@@ -26,7 +26,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kChunk = 256;              // consecutive slots a warp takes at a time
-constexpr unsigned kWarpSortMax = 512;   // longest row a warp sorts in registers
+constexpr unsigned kWarpSortMax = kMidRow;   // longest row a warp sorts in registers
 constexpr unsigned kStage = 1024;        // pairs a warp stages in shared memory
 constexpr unsigned kRankMax = 64;        // longest row ranked by counting
 
@@ -85,10 +85,10 @@ __global__ void fill_u32(uint32_t* p, size_t n, uint32_t v) {
 
 // Step 1.  kDirected: both directions of every (i < j) key (the self pairs are in the initial counts).
 template <bool kDirected>
-__global__ void __launch_bounds__(kThreads) row_count(const uint64_t* keys, const unsigned long long* reserved,
-                                                      unsigned long long cap, const RowTables t, uint32_t nrows,
-                                                      uint32_t* cnt) {
-    const unsigned long long n = min(*reserved, cap);
+__global__ void __launch_bounds__(kThreads) row_count(const uint64_t* keys, const Counters* ctr, unsigned long long cap,
+                                                      const RowTables t, uint32_t nrows, uint32_t* cnt) {
+    const unsigned long long n = ctr->acc_reserved, pairs = ctr->acc_valid;
+    if (n > cap || !rows_may_fit(kDirected ? 2 * pairs + nrows : pairs, nrows)) return;   // as the host reads them
     const unsigned lane = lane_id();
     const unsigned long long nw = (unsigned long long)gridDim.x * kWarps;
     int hint = 0;
@@ -448,9 +448,8 @@ RowTable make_row_table(unsigned long long key_off, unsigned long long row_off, 
     return RowTable{key_off, row_off, std::max(n_cols, 1ull), n_cols > 1 ? ~0ull / n_cols : ~0ull};
 }
 
-void count_rows(const uint64_t* keys, const Counters* ctr, unsigned long long cap, const RowTables& t, bool directed,
-                uint32_t nrows, uint32_t* cnt, uint32_t* first, unsigned long long* longest, uint32_t* ws,
-                cudaStream_t st) {
+void count_rows(const uint64_t* keys, Counters* ctr, unsigned long long cap, const RowTables& t, bool directed,
+                uint32_t nrows, uint32_t* cnt, uint32_t* first, uint32_t* ws, cudaStream_t st) {
     if (directed)   // every row's self pair
         launch(fill_u32, std::max(1u, std::min((nrows + 255) / 256, (unsigned)num_sms() * 8)), 256, 0, st, cnt,
                (size_t)nrows, 1u);
@@ -458,10 +457,11 @@ void count_rows(const uint64_t* keys, const Counters* ctr, unsigned long long ca
         TJ_CUDA(cudaMemsetAsync(cnt, 0, (size_t)nrows * sizeof(uint32_t), st));
     const unsigned blocks = slot_blocks(cap);
     if (directed)
-        launch(row_count<true>, blocks, kThreads, 0, st, keys, &ctr->acc_reserved, cap, t, nrows, cnt);
+        launch(row_count<true>, blocks, kThreads, 0, st, keys, (const Counters*)ctr, cap, t, nrows, cnt);
     else
-        launch(row_count<false>, blocks, kThreads, 0, st, keys, &ctr->acc_reserved, cap, t, nrows, cnt);
-    exclusive_scan_u32(cnt, first, nrows, nullptr, ws, st, longest);
+        launch(row_count<false>, blocks, kThreads, 0, st, keys, (const Counters*)ctr, cap, t, nrows, cnt);
+    static_assert(offsetof(Counters, long_pairs) == offsetof(Counters, longest_row) + 8, "the scan's two words");
+    exclusive_scan_u32(cnt, first, nrows, nullptr, ws, st, &ctr->longest_row);
 }
 
 void order_rows(const uint64_t* keys, unsigned long long slots, const RowTables& t, bool directed, uint32_t nrows,

@@ -23,13 +23,19 @@ constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
 constexpr size_t kScanOne = 4 * kScanTile;   // up to here one block scans everything
 
-TJ_DEV uint32_t load_items(const uint32_t* in, size_t base, size_t n, uint32_t (&v)[kScanItems], uint32_t& most) {
+// What a thread saw of the elements: the largest, and the sum of those above kMidRow.
+struct Lengths {
+    uint32_t most = 0;
+    unsigned long long above = 0;
+};
+TJ_DEV uint32_t load_items(const uint32_t* in, size_t base, size_t n, uint32_t (&v)[kScanItems], Lengths& len) {
     uint32_t local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         v[k] = (base + k < n) ? in[base + k] : 0u;
         local += v[k];
-        most = max(most, v[k]);
+        len.most = max(len.most, v[k]);
+        len.above += v[k] > kMidRow ? v[k] : 0u;
     }
     return local;
 }
@@ -53,48 +59,57 @@ TJ_DEV void store_items(uint32_t* out, size_t base, size_t n, uint32_t run, cons
         run += v[k];
     }
 }
-TJ_DEV void raise_longest(unsigned long long* longest, uint32_t most) {
-    if (!longest) return;
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (lane_id() == 0 && most) atomicMax(longest, (unsigned long long)most);
+TJ_DEV void add_lengths(unsigned long long* lengths, const Lengths& len) {
+    if (!lengths) return;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, len.most);
+    if (most == 0) return;   // warp-uniform
+    unsigned long long above = len.above;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+    if (lane_id() != 0) return;
+    atomicMax(lengths, (unsigned long long)most);
+    if (above) atomicAdd(lengths + 1, above);
 }
 
 // Short arrays: one block, tile after tile.
 __global__ void __launch_bounds__(kScanThreads) scan_one(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total,
-                                                         unsigned long long* longest) {
+                                                         unsigned long long* lengths) {
     __shared__ uint32_t warp_tot[32];
-    uint32_t carry = 0, most = 0;
+    uint32_t carry = 0;
+    Lengths len;
     for (size_t t = 0; t < n; t += kScanTile) {
         const size_t base = t + (size_t)threadIdx.x * kScanItems;
         uint32_t v[kScanItems], all;
-        const uint32_t local = load_items(in, base, n, v, most);
+        const uint32_t local = load_items(in, base, n, v, len);
         const uint32_t pre = block_scan(local, warp_tot, all);
         store_items(out, base, n, carry + pre, v);
         carry += all;
     }
     if (total && threadIdx.x == 0) *total = carry;
-    raise_longest(longest, most);
+    add_lengths(lengths, len);
 }
 
 // Longer arrays: the tiles' sums, then every tile adds up the sums before it and scans itself.
 __global__ void __launch_bounds__(kScanThreads) scan_sums(const uint32_t* in, size_t n, uint32_t* sums,
-                                                          unsigned long long* longest) {
+                                                          unsigned long long* lengths) {
     __shared__ uint32_t warp_tot[32];
-    uint32_t v[kScanItems], most = 0, all;
+    uint32_t v[kScanItems], all;
+    Lengths len;
     const uint32_t local =
-        load_items(in, (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems, n, v, most);
+        load_items(in, (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems, n, v, len);
     block_scan(local, warp_tot, all);
     if (threadIdx.x == 0) sums[blockIdx.x] = all;
-    raise_longest(longest, most);
+    add_lengths(lengths, len);
 }
 __global__ void __launch_bounds__(kScanThreads) scan_apply(const uint32_t* in, uint32_t* out, size_t n,
                                                            const uint32_t* sums, uint32_t* total) {
     __shared__ uint32_t warp_tot[32];
-    uint32_t part = 0, before, all, v[kScanItems], most = 0;
+    uint32_t part = 0, before, all, v[kScanItems];
+    Lengths len;
     for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads) part += sums[b];
     block_scan(part, warp_tot, before);
     const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-    const uint32_t local = load_items(in, base, n, v, most);
+    const uint32_t local = load_items(in, base, n, v, len);
     const uint32_t pre = block_scan(local, warp_tot, all);
     store_items(out, base, n, before + pre, v);
     if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + all;
@@ -109,17 +124,17 @@ size_t scan_workspace_elems(size_t n) { return (n + kScanTile - 1) / kScanTile +
 // elements, two above (the recursive form it replaces took three to six, and small joins are bound by
 // the number of launches).
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
-                        cudaStream_t st, unsigned long long* longest) {
+                        cudaStream_t st, unsigned long long* lengths) {
     if (n == 0) {
         if (total) TJ_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), st));
         return;
     }
     if (n <= kScanOne) {
-        launch(scan_one, 1, kScanThreads, 0, st, in, out, n, total, longest);
+        launch(scan_one, 1, kScanThreads, 0, st, in, out, n, total, lengths);
         return;
     }
     const unsigned nb = (unsigned)((n + kScanTile - 1) / kScanTile);
-    launch(scan_sums, nb, kScanThreads, 0, st, in, n, ws, longest);
+    launch(scan_sums, nb, kScanThreads, 0, st, in, n, ws, lengths);
     launch(scan_apply, nb, kScanThreads, 0, st, in, out, n, (const uint32_t*)ws, total);
 }
 
