@@ -103,7 +103,9 @@ typedef struct tj_options {
  * every pair exactly inside the screen (no band).  By default, for rows of up to 256 elements, the
  * screen issues only the high-limb product hh, bounds the low-limb terms by Cauchy-Schwarz, decides
  * each candidate by an exact INT64 interval test, and sends the few undecided pairs to the exact
- * integer refinement (tj_stats.band).  The pairs are the same either way. */
+ * integer refinement (tj_stats.band); where that leaves more than a sixteenth of the pairs undecided
+ * (rows of small values) the join goes over to all four products by itself (one more of
+ * tj_stats.retries).  The pairs are the same either way. */
 #define TJ_FLAG_I8_FOUR_PRODUCTS 32
 /* Guard regions: 512 words of a fixed pattern (every byte -17, the reference's fill for retained
  * buffers) right after the part of the accept, band, result-key and sort buffers that a stage may

@@ -691,7 +691,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
 
     // candidate tile pairs (block-diagonal over joins) and execution chunks
     // the int8 high-limb screen takes R tiles in groups, and chunks short enough that every SM gets several
-    const int rgroup = i8 && i8_high_limb_screen(g) ? i8_rtiles(C[0]->R.kpad / 128) : 1;
+    int rgroup = i8 && i8_high_limb_screen(g) ? i8_rtiles(C[0]->R.kpad / 128) : 1;
     if (rgroup > 1 && !(opt && opt->chunk_items > 0)) {
         const long long lists = (g.ntR_total + rgroup - 1) / rgroup, entries = lists * g.ntS_total / (self ? 2 : 1);
         chunk_items = (int)std::min(64ll, std::max(4ll, entries / (num_sms() * 6) / 2 * 2));
@@ -773,10 +773,13 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         }
         half_masks(hv, cand, g.ntR_total, d_rt.p, d_jps.p, self, full, st);
     }
-    launch(pairs_screened_kernel, num_sms() * 4, 256, 0, st, (const uint4*)cand.chunks.p,
-           (const uint32_t*)(cand.dev_counts.p + 1), (const uint32_t*)cand.jlist.p, (const uint4*)d_rt.p,
-           (const uint4*)d_st.p, sops, g.half_packed ? 1 : 0, rgroup,
-           &ctr.p->pairs_screened);
+    auto count_screened = [&] {
+        launch(pairs_screened_kernel, num_sms() * 4, 256, 0, st, (const uint4*)cand.chunks.p,
+               (const uint32_t*)(cand.dev_counts.p + 1), (const uint32_t*)cand.jlist.p, (const uint4*)d_rt.p,
+               (const uint4*)d_st.p, sops, g.half_packed ? 1 : 0, rgroup,
+               &ctr.p->pairs_screened);
+    };
+    count_screened();
     ev.rec(6, st);
 
     // optional screen-error sampling (tensor-core screens): 64 tile pairs spread over the candidate list
@@ -880,6 +883,20 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         if (!over) break;
         if (attempt >= 6) fail(TJ_ERR_NOMEM, "output capacity retries exhausted");
         S_.retries++;
+        if (i8 && i8_high_limb_screen(g) && h.band_reserved > i8_band_stop(h.pairs_screened, bcap)) {
+            // too many pairs undecided by the high limbs: four products, over lists of single R tiles
+            g.i8_four_products = true;
+            rgroup = 1;
+            chunk_items = (opt && opt->chunk_items > 0) ? opt->chunk_items : 64;
+            cand = Candidates();
+            build_candidates(*g.tR[0], *g.tS[0], jps[0].Tp, self, chunk_items, cand, st, rgroup);
+            sops.per_item[0] = 2.0 * kTileR * 128.0 * (double)C[0]->R.kpad * 0.5;
+            TJ_CUDA(cudaMemsetAsync(&ctr.p->pairs_screened, 0,
+                                    offsetof(Counters, screen_reserved) - offsetof(Counters, pairs_screened), st));
+            count_screened();
+            if (h.acc_reserved > cap) cap = std::max(cap * 2, h.acc_reserved + h.acc_reserved / 4 + 4096);
+            continue;
+        }
         cap = std::max(cap * 2, h.acc_reserved + h.acc_reserved / 4 + 4096);
         bcap = std::max(bcap * 2, h.band_reserved + h.band_reserved / 4 + 4096);
     }

@@ -330,6 +330,15 @@ struct ScreenInput {
 void screen_tc(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st);
 void screen_plain(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st);
 void screen_i8(const ScreenInput& g, const EmitBuffers& eb, cudaStream_t st);
+// Band slots from which on the high-limb screen is given up for the four-product one: more than a sixteenth of
+// the pairs (of 2^20 at least) undecided, as on rows of small values, whose high limbs say next to nothing.
+// 20,000 rows of values up to 8 ... 300: whole join with four products 2.4 to 2.7 ms, where the band and its
+// refinement took 4 to 38 ms; up to 1,000 (1 to 50 % of the pairs) 1.0 to 2.6 against 1.3 to 27; up to 3,000
+// (below 2 %) 0.8 to 1.7 against 0.5 to 2.2.
+__host__ __device__ inline unsigned long long i8_band_stop(unsigned long long pairs_screened, unsigned long long band_cap) {
+    const unsigned long long least = band_cap > (1ull << 20) ? band_cap : 1ull << 20;
+    return pairs_screened >> 4 > least ? pairs_screened >> 4 : least;
+}
 // true when screen_i8 runs the high-limb screen (hh products only; undecided pairs go to the band
 // and the exact integer refinement), false for the four-product screen (exact, no band)
 bool i8_high_limb_screen(const ScreenInput& g);

@@ -835,12 +835,15 @@ __global__ void __launch_bounds__(kHHThreads, 1)
             // list entries 32 at a time, the next 32 on their way
             unsigned eb = ch.y;
             uint32_t cur = a.jlist[min(eb + lane, ch.z - 1)], nxt = a.jlist[min(eb + 32 + lane, ch.z - 1)];
-            // floor((A_i - T) / 2^15) of this lane's row of every R tile (no point: rejects everything)
+            // floor((A_i - T) / 2^15) of this lane's row of every R tile (no point: rejects everything; the same
+            // once the join is to be done with four products instead, as the host will see by the counter)
+            const bool given_up = *(volatile unsigned long long*)&a.ctr->band_reserved >
+                                  i8_band_stop(a.ctr->pairs_screened, a.band_cap);
             int c15[kRT];
 #pragma unroll
             for (unsigned r = 0; r < (unsigned)kRT; ++r) {
                 const unsigned gr = (ch.x * kRT + r) * 128 + row;
-                c15[r] = gr < a.nR ? clamp_shift15(a.rrec[gr].norm - a.T) : 0x7FFFFFFF;
+                c15[r] = gr < a.nR && !given_up ? clamp_shift15(a.rrec[gr].norm - a.T) : 0x7FFFFFFF;
             }
             for (unsigned e = ch.y; e < ch.z && ok; e += 2) {
                 if (e - eb == 32) {
