@@ -59,7 +59,8 @@ extern "C" {
 #define TJ_SCREEN_BF16X3 4      /* BF16 hi + lo operand limbs, 3 products per k into one FP32 accumulator */
 #define TJ_SCREEN_FP16X3 5      /* FP16 hi + lo operand limbs, 3 products per k into one FP32 accumulator */
 
-/* A small join without options (rows of at most 192 elements, pairs x (d + 8) at most 2^31) is done
+/* A small join without options (rows of at most 192 elements, |R| at most 2^15 and |S| 2^20, pairs x (d + 8)
+ * at most 2^31, and 2^32 with |R| counted in whole tiles of 128; half of the pairs in upper mode) is done
  * directly whatever float screen is named: FP32 direct differences of every pair, FP64 for those they
  * leave open.  The pairs, and what is refused, are those of the named screen; tj_stats describes what
  * ran (all pairs screened, no index or candidate stage).  Any option selects the indexed path. */

@@ -1,11 +1,12 @@
 // C ABI of libtensorjoin: orchestration of index -> candidates -> screen -> refine -> sort.
 //
-// One host synchronisation per join: after the screen and the refinement the
-// counters are read back once to size the output (and to detect a capacity
+// The host waits twice in a join: after the screen and the refinement the
+// counters are read back to size the output (and to detect a capacity
 // overflow, in which case both stages run again with larger buffers -- the
-// overflow-and-retry pass of the reference, src/run_g2a_tensorjoin.py:329-378).
-// Everything else stays on the device in stream order; memory comes from a
-// private stream-ordered pool so repeated joins do not hit cudaMalloc.
+// overflow-and-retry pass of the reference, src/run_g2a_tensorjoin.py:329-378),
+// and at the end for the status of the ordering.  Everything else stays on the
+// device in stream order; memory comes from a private stream-ordered pool so
+// repeated joins do not hit cudaMalloc.
 #include <algorithm>
 #include <chrono>
 #include <atomic>
@@ -843,7 +844,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     }
     Counters h;
     for (int attempt = 0;; ++attempt) {
-        acc = DBuf<uint64_t>::result(cap + gs, st);   // becomes the result's key array
+        acc = DBuf<uint64_t>::result(cap + gs, st);   // a result by whole keys may keep it
         band = DBuf<uint64_t>(bcap + gs, st);
         launch(zero_counters, 1, 32, 0, st, ctr.p, 1);
         if (times) {   // first starts: all ones (atomicMin), last ends and CTA stamps: zero

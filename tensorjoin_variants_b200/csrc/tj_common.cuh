@@ -405,10 +405,6 @@ __host__ __device__ constexpr uint32_t desc_hi_for_rows(unsigned row_bytes) {
     return ((8u * row_bytes) >> 4) | (1u << 14) |
            ((row_bytes == 32u ? 6u : row_bytes == 64u ? 4u : 2u) << 29);
 }
-TJ_DEV uint64_t desc_kmajor(const void* smem_base, unsigned byte_off, uint32_t desc_hi) {
-    const unsigned a = smem_u32(smem_base) + byte_off;
-    return ((uint64_t)desc_hi << 32) | (uint64_t)(1u << 16) | (uint64_t)((a >> 4) & 0x3FFFu);
-}
 
 // UMMA instruction descriptor (kind::f16 / kind::i8, dense, K-major A and B).
 // a/b format: f16 = 0, bf16 = 1 (kind::f16); u8 = 0, s8 = 1 (kind::i8).  c format: f32 = 1, s32 = 2.

@@ -55,9 +55,9 @@ TJ_DEV double seq_d2(const float* x, const float* y, int d) {
 //
 // What bounds it: FP32 issue (a packed subtract and a packed FMA per two elements of a pair; the
 // packed pipe alone needs 180 us for the 202M pairs of a 20,000 x 16 self-join), with the per-pair
-// sum and classification on top of it below d = 16.  The form this replaces took 31,000 cycles per
-// 128 x 256 tile pair at d = 16 and at d = 2 alike (8 x 16 pairs per thread and one CTA per SM: the
-// latency of unpipelined loads and a branch per pair).  Hence two CTAs of 8 warps per SM, operand
+// sum and classification on top of it below d = 16.  With 8 x 16 pairs per thread, one CTA per SM,
+// unpipelined loads and a branch per pair it was latency: 31,000 cycles per 128 x 256 tile pair at d = 16
+// and at d = 2 alike.  Hence two CTAs of 8 warps per SM, operand
 // chunks brought in two stages ahead by cp.async (across unit and tile borders), one minimum over a
 // thread's 32 pairs in front of the per-pair tests, and an even cut of all units over the CTAs
 // (chunks of 64 tile pairs left half of them idle on 20,000 rows).  Measured (one B200): 20,000 x 16

@@ -514,10 +514,9 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 // in the accumulator (norms in units of sqrt(128), rounded up), and v < floor((A_i - T) / 2^15) proves
 // the pair out: one maximum per row over any number of columns, against a constant of the row.
 //
-// What bounds it.  The form this replaces (a 128 x 128 item per step, group tests against column norms,
-// metadata and an FP64 row bound per item) took 1,300 cycles per item where its MMAs need 256.  Builds
-// that skip work showed why, one limit behind the other:
-//  - the S limbs streamed from L2, 20 KB per item and 7 TB/s in all: a CTA now holds kRT R tiles and
+// What bounds it.  A 128 x 128 item needs 256 cycles of MMAs and took 1,300 with one R tile per CTA and
+// per-column tests.  Builds that skip work showed why, one limit behind the other:
+//  - the S limbs streamed from L2, 20 KB per item and 7 TB/s in all: a CTA holds kRT R tiles and
 //    every S tile brought in meets all of them;
 //  - the issuing thread's own instructions, 700 cycles per step with one MMA in it: two S tiles share
 //    an N = 256 MMA (and a commit, two barriers and each A fragment read), loops are unrolled, and a
@@ -528,7 +527,8 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 // Now (cycles per item at 1M rows): MMAs and copies alone 420, with the epilogue's tests 600, with the
 // candidates of a 24-neighbour threshold 775.
 // Candidates come as lists per group of kRT R tiles whose entries say which of them they are for.
-// Measured (one B200, 24 neighbours per row, self-join): 2M x 128 554 -> 335 ms, 50,021 x 100 1.00 -> 0.57 ms.
+// Measured (one B200, self-joins with 24 neighbours per row, this kernel alone): 2M x 128 554 -> 335 ms,
+// 50,021 x 100 1.00 -> 0.57 ms.
 //
 // Warp roles (512 threads): warps 0 and 2 TMA producers (limbs; folds), warp 1 TMEM
 // allocator + UMMA issuer, warp 3 idle, warps 4..15 epilogue in three groups of four that take the live 128 x 128 items in turn (warp w

@@ -121,8 +121,7 @@ size_t scan_workspace_elems(size_t n) { return (n + kScanTile - 1) / kScanTile +
 
 // out[i] = sum_{k<i} in[k]; optional *total = sum of all (device pointer).
 // `ws` needs scan_workspace_elems(n) u32 elements.  `in` and `out` may alias.  One launch up to 16,384
-// elements, two above (the recursive form it replaces took three to six, and small joins are bound by
-// the number of launches).
+// elements, two above: small joins are bound by the number of launches.
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, uint32_t* ws,
                         cudaStream_t st, unsigned long long* lengths) {
     if (n == 0) {
