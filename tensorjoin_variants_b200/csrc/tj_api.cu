@@ -67,8 +67,8 @@ void stage_reset() {
     for (auto& c : g_stage) c.used = 0;
 }
 
-void upload(void* dev_dst, const void* host_src, size_t bytes, cudaStream_t st) {
-    if (bytes == 0) return;
+// Pinned host memory of the calling thread, until the next stage_reset.
+static uint8_t* stage_take(size_t bytes) {
     const size_t need = (bytes + 255) & ~(size_t)255;
     StageChunk* ch = nullptr;
     for (auto& c : g_stage)
@@ -80,8 +80,14 @@ void upload(void* dev_dst, const void* host_src, size_t bytes, cudaStream_t st) 
         g_stage.push_back(c);
         ch = &g_stage.back();
     }
-    uint8_t* src = ch->p + ch->used;
+    uint8_t* p = ch->p + ch->used;
     ch->used += need;
+    return p;
+}
+
+void upload(void* dev_dst, const void* host_src, size_t bytes, cudaStream_t st) {
+    if (bytes == 0) return;
+    uint8_t* src = stage_take(bytes);
     memcpy(src, host_src, bytes);
     TJ_CUDA(cudaMemcpyAsync(dev_dst, src, bytes, cudaMemcpyHostToDevice, st));
     if (!g_stage_done) TJ_CUDA(cudaEventCreateWithFlags(&g_stage_done, cudaEventDisableTiming));
@@ -842,7 +848,8 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         rows = DBuf<uint32_t>::result(rows_even + guard32, st);
         rows_ws = DBuf<uint32_t>(scan_workspace_elems(nrows), st);
     }
-    Counters h;
+    // (both read-backs go to pinned memory: to pageable memory each costs 10 us)
+    Counters& h = *(Counters*)stage_take(sizeof(Counters));
     for (int attempt = 0;; ++attempt) {
         acc = DBuf<uint64_t>::result(cap + gs, st);   // a result by whole keys may keep it
         band = DBuf<uint64_t>(bcap + gs, st);
@@ -1046,7 +1053,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
     }
     ev.rec(5, st);
     // what the ordering found (a key outside the rows, a look-back that gave up, an overwritten guard)
-    unsigned long long status_after = 0;
+    unsigned long long& status_after = *(unsigned long long*)stage_take(8);
     TJ_CUDA(cudaMemcpyAsync(&status_after, &ctr.p->status, 8, cudaMemcpyDeviceToHost, st));
     TJ_CUDA(cudaStreamSynchronize(st));
     check_status(status_after);
