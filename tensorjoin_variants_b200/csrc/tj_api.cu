@@ -848,7 +848,7 @@ void run_batch_body(const std::vector<JoinIn>& joins, int dtype, int mode, int s
         rows = DBuf<uint32_t>::result(rows_even + guard32, st);
         rows_ws = DBuf<uint32_t>(scan_workspace_elems(nrows), st);
     }
-    // (both read-backs go to pinned memory: to pageable memory each costs 10 us)
+    // (this and the status at the end are read back to pinned memory: 20,000 x 16 self-join 710 -> 702 us)
     Counters& h = *(Counters*)stage_take(sizeof(Counters));
     for (int attempt = 0;; ++attempt) {
         acc = DBuf<uint64_t>::result(cap + gs, st);   // a result by whole keys may keep it
